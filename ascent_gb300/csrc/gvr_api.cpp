@@ -435,7 +435,7 @@ static void free_domain(Domain &d)
 {
   cudaFree(d.d_bricks);
   cudaFree(d.d_cells);
-  for (int a = 0; a < 3; ++a) cudaFree(d.d_coord[a]);
+  cudaFree(d.d_cell_rec);
   cudaFree(d.d_brick_range);
   cudaFree(d.d_brick_empty);
   cudaFree(d.stg.buf);
@@ -556,26 +556,47 @@ static int add_structured(gvr_scene *s, int kind, const int dims[3], const doubl
       d.bounds[2 * a + 1] = d.dev.hi[a];
     }
   } else {
+    // a vertex field's brick offset is linear in the axes' bricks and places,
+    // so each axis adds its share
+    std::vector<RectCell> rec;
+    const int sh = s->brick_shift;
+    int64_t in_brick = 1, of_brick = brick_floats(sh);
     for (int a = 0; a < 3; ++a) {
       if (!coords[a]) return set_error(GVR_ERR_INVALID_ARGUMENT, "rectilinear coordinates are NULL");
-      std::vector<float> c(dims[a]);
-      for (int i = 0; i < dims[a]; ++i) {
-        c[i] = (float)coords[a][i];
-        if (i > 0 && !(c[i] > c[i - 1]))
+      const int n = dims[a] - 1;
+      const size_t first = rec.size();
+      rec.resize(first + 2 * (size_t)n);
+      float x0 = (float)coords[a][0];
+      d.dev.lo[a] = x0;
+      for (int i = 0; i < n; ++i) {
+        const float x1 = (float)coords[a][i + 1];
+        if (!(x1 > x0))
           return set_error(GVR_ERR_INVALID_ARGUMENT, "rectilinear coordinates must increase");
+        RectCell &f = rec[first + i];
+        f.x0 = x0;
+        f.width = x1 - x0;
+        f.inv_width = 1.0f / f.width;
+        f.ahead = i + 1 < n ? x1 : INFINITY;
+        f.share = assoc == GVR_ASSOC_ELEMENT
+                      ? i : (int)((i >> sh) * of_brick + (i & (brick_cells(sh) - 1)) * in_brick);
+        rec[first + n + i] = f;
+        rec[first + n + i].ahead = i > 0 ? -x0 : INFINITY;
+        x0 = x1;
       }
-      e = cudaMalloc(&d.d_coord[a], sizeof(float) * dims[a]);
-      if (e != cudaSuccess) { free_domain(d); return cuda_error(e, "cudaMalloc coords"); }
-      e = cudaMemcpy(d.d_coord[a], c.data(), sizeof(float) * dims[a], cudaMemcpyHostToDevice);
-      if (e != cudaSuccess) { free_domain(d); return cuda_error(e, "copy coords"); }
-      d.dev.coord[a] = d.d_coord[a];
-      d.dev.lo[a] = c.front();
-      d.dev.hi[a] = c.back();
-      d.dev.origin[a] = c.front();
+      in_brick *= brick_nodes(sh);
+      of_brick *= d.dev.nbrick[a];
+      d.dev.rec_first[a] = (int)first;
+      d.dev.hi[a] = x0;
+      d.dev.origin[a] = d.dev.lo[a];
       d.dev.inv_spacing[a] = 1.f;
-      d.bounds[2 * a] = c.front();
-      d.bounds[2 * a + 1] = c.back();
+      d.bounds[2 * a] = d.dev.lo[a];
+      d.bounds[2 * a + 1] = d.dev.hi[a];
     }
+    e = cudaMalloc(&d.d_cell_rec, sizeof(RectCell) * rec.size());
+    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc coords");
+    e = cudaMemcpy(d.d_cell_rec, rec.data(), sizeof(RectCell) * rec.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) { free_domain(d); return cuda_error(e, "copy coords"); }
+    d.dev.cell_rec = d.d_cell_rec;
   }
   if (assoc == GVR_ASSOC_VERTEX) {
     d.n_values = (size_t)dims[0] * dims[1] * dims[2];
@@ -1015,6 +1036,17 @@ static int prepare_march(gvr_scene *s, const gvr_render_params *p, cudaStream_t 
   return GVR_OK;
 }
 
+// Which march kernel the scene's domains need.
+static int march_mode(const gvr_scene *s)
+{
+  int mode = s->has_hex ? kMarchHex : kMarchUniform;
+  for (const Domain &d : s->domains) {
+    if (d.dev.kind == GVR_DOMAIN_RECTILINEAR) mode = std::max<int>(mode, kMarchRect);
+    else if (d.dev.assoc != GVR_ASSOC_VERTEX) mode = std::max<int>(mode, kMarchCells);
+  }
+  return mode;
+}
+
 static int render_one(gvr_scene *s, const gvr_camera *camera, const gvr_render_params *p,
                       float *rgba, float *depth, int out_location, void *stream,
                       uint64_t *samples_out, bool over);
@@ -1249,7 +1281,7 @@ static int render_one(gvr_scene *s, const gvr_camera *camera, const gvr_render_p
                       s->d_counters + 1, st);
   } else {
     e = launch_march(s->d_domains, view, mp, s->d_lut, d_rgba, d_depth,
-                     samples_out ? s->d_counters : nullptr, s->tuning, s->has_hex, d_order, st);
+                     samples_out ? s->d_counters : nullptr, s->tuning, march_mode(s), d_order, st);
   }
   if (e != cudaSuccess) return cuda_error(e, "march kernel launch");
   if (out_location == GVR_MEM_HOST) {
@@ -1379,7 +1411,7 @@ int gvr_render_volume_batch(gvr_scene *s, const gvr_camera *cameras, int n_views
   // once per launch configuration and replayed as a CUDA graph.
   struct Key {
     MarchParams mp;
-    int n_views, packet_w, unroll, min_blocks, tpi, has_hex;
+    int n_views, packet_w, unroll, min_blocks, tpi, mode;
     const void *ptrs[6];
   } key;
   std::memset(static_cast<void *>(&key), 0, sizeof(key));  // padding too: compared bytewise
@@ -1389,7 +1421,7 @@ int gvr_render_volume_batch(gvr_scene *s, const gvr_camera *cameras, int n_views
   key.unroll = s->tuning.unroll;
   key.min_blocks = s->tuning.min_blocks;
   key.tpi = s->tuning.tiles_per_item;
-  key.has_hex = s->has_hex ? 1 : 0;
+  key.mode = march_mode(s);
   const void *ptrs[6] = {d_rgba, d_depth, d_samples, s->d_views, s->d_rects, s->d_domains};
   std::memcpy(key.ptrs, ptrs, sizeof(ptrs));
   const unsigned char *kb = reinterpret_cast<const unsigned char *>(&key);
@@ -1400,13 +1432,13 @@ int gvr_render_volume_batch(gvr_scene *s, const gvr_camera *cameras, int n_views
       s->batch_exec = nullptr;
     }
     int grid = 0;
-    if ((e = batch_grid(mp, n_views, s->tuning, s->has_hex, &grid)) != cudaSuccess)
+    if ((e = batch_grid(mp, n_views, s->tuning, key.mode, &grid)) != cudaSuccess)
       return cuda_error(e, "batch launch shape");
     cudaGraph_t graph = nullptr;
     e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_error(e, "cudaStreamBeginCapture");
     cudaError_t le = launch_batch(s->d_domains, s->d_views, s->d_rects, mp, n_views, s->d_lut, d_rgba,
-                                  d_depth, d_samples, s->d_queue, s->tuning, s->has_hex, grid, st);
+                                  d_depth, d_samples, s->d_queue, s->tuning, key.mode, grid, st);
     e = cudaStreamEndCapture(st, &graph);
     if (le != cudaSuccess) { if (graph) cudaGraphDestroy(graph); return cuda_error(le, "batch capture"); }
     if (e != cudaSuccess) return cuda_error(e, "cudaStreamEndCapture");

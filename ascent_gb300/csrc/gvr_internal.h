@@ -37,7 +37,21 @@ static_assert(brick_floats(kBrickShiftDefault) == kBrickFloats, "default brick")
 
 constexpr int kMaxDomains = 64;     // domains a single render can composite
 constexpr int kMaxLut = 4096;
+// What a scene's domains are, for the choice of a march kernel (each carries
+// the march code of those before it too): uniform grids with vertex fields
+// alone; uniform grids; structured grids; hexahedra among them.
+enum { kMarchUniform = 0, kMarchCells = 1, kMarchRect = 2, kMarchHex = 3 };
 constexpr int kMarchTile = 16;      // march kernel: one CTA per 16x16-pixel tile
+
+// A cell of a rectilinear domain's axis, for rays in one of its directions:
+// first node, width and 1 / width; the node ahead times the direction's sign
+// (infinite in the last cell); the cell's share of a vertex field's brick
+// offset, or its own index for a cell-centred field. An axis of n cells has n
+// records for rays along it, then n for rays against it.
+struct alignas(32) RectCell {
+  float x0, width, inv_width, ahead;
+  int share;
+};
 
 // Device view of one structured domain.
 struct DomainDev {
@@ -51,7 +65,8 @@ struct DomainDev {
   int assoc;              // GVR_ASSOC_VERTEX / ELEMENT
   const float *bricks;    // vertex fields: bricked nodes
   const float *cells;     // element fields: linear cell values
-  const float *coord[3];  // rectilinear node coordinates
+  const RectCell *cell_rec;   // rectilinear: the axes' cells (see RectCell)
+  int rec_first[3];           // axis a's forward records, from cell_rec[rec_first[a]]
   const float2 *brick_range;  // per-brick {min, max} of the field
   const uint8_t *brick_empty; // per-brick 1 = LUT alpha is 0 over its range
   const int *any_empty;       // 1 if any brick of this domain is empty
@@ -137,7 +152,7 @@ struct Domain {
   size_t n_values = 0;             // field values
   float *d_bricks = nullptr;
   float *d_cells = nullptr;
-  float *d_coord[3] = {nullptr, nullptr, nullptr};
+  RectCell *d_cell_rec = nullptr;
   float2 *d_brick_range = nullptr;
   uint8_t *d_brick_empty = nullptr;
   int64_t n_bricks = 0;
@@ -297,7 +312,7 @@ cudaError_t launch_march(const DomainDev *d_domains, const ViewDev &view,
                          const MarchParams &mp, const float4 *d_lut,
                          float4 *d_rgba, float *d_depth,
                          unsigned long long *d_samples, const Tuning &tuning,
-                         bool has_hex, const int *d_order, cudaStream_t stream);
+                         int mode, const int *d_order, cudaStream_t stream);
 // longest-first tile order for one view (gvr_march.cu): writes a permutation
 // of the view's kMarchTile tiles to d_order (one int per tile); d_keys holds
 // one word per tile of scratch and *d_top a word that is 0 between calls;
@@ -313,11 +328,11 @@ cudaError_t launch_staged(const DomainDev *d_domains, const ViewDev &view, const
                           unsigned long long *d_samples, const Tuning &tuning, const int *d_order,
                           const StageOrder &order, unsigned long long *d_stage_fail,
                           cudaStream_t stream);
-cudaError_t batch_grid(const MarchParams &mp, int n_views, const Tuning &tuning, bool has_hex,
+cudaError_t batch_grid(const MarchParams &mp, int n_views, const Tuning &tuning, int mode,
                        int *grid);
 cudaError_t launch_batch(const DomainDev *d_domains, const ViewDev *d_views, const int4 *d_rects,
                          const MarchParams &mp, int n_views, const float4 *d_lut, float4 *d_rgba,
                          float *d_depth, unsigned long long *d_samples, unsigned int *d_queue,
-                         const Tuning &tuning, bool has_hex, int grid, cudaStream_t stream);
+                         const Tuning &tuning, int mode, int grid, cudaStream_t stream);
 
 }  // namespace gvr
