@@ -250,7 +250,16 @@ void make_view(const gvr_camera &cam, int width, int height, ViewDev *v)
       M[i * 4 + j] = acc;
       v->projview[i * 4 + j] = (float)acc;
     }
-  invert4(M, v->inv_projview);
+  double inv[16];
+  invert4(M, inv);
+  for (int i = 0; i < 4; ++i) {
+    const double *q = inv + 4 * i;
+    const double row[4] = {q[0] * 2 / width, q[1] * 2 / height, q[2] * 2, q[3] - q[0] - q[1] - q[2]};
+    for (int j = 0; j < 4; ++j) {
+      v->unproject[4 * i + j] = row[j];
+      v->unproject_f[4 * i + j] = (float)row[j];
+    }
+  }
 }
 
 }  // namespace gvr
@@ -1281,7 +1290,8 @@ static int render_one(gvr_scene *s, const gvr_camera *camera, const gvr_render_p
                       s->d_counters + 1, st);
   } else {
     e = launch_march(s->d_domains, view, mp, s->d_lut, d_rgba, d_depth,
-                     samples_out ? s->d_counters : nullptr, s->tuning, march_mode(s), d_order, st);
+                     samples_out ? s->d_counters : nullptr, s->tuning, std::max<int>(march_mode(s), over ? kMarchCells : kMarchUniform),
+                     d_order, st);
   }
   if (e != cudaSuccess) return cuda_error(e, "march kernel launch");
   if (out_location == GVR_MEM_HOST) {

@@ -111,7 +111,11 @@ struct ViewDev {
   float xoff;             // pan, in pixels
   float yoff;
   float projview[16];     // row-major projection * view (image depth)
-  double inv_projview[16]; // its inverse (opaque canvas depth -> distance)
+  // pixel (i, j) and canvas depth d -> homogeneous world point: the inverse
+  // of projview behind the NDC map (2i/W - 1, 2j/H - 1, 2d - 1); in FP32 too,
+  // for the bound that tells where a canvas can end a ray
+  double unproject[16];
+  float unproject_f[16];
 };
 
 struct MarchParams {

@@ -626,28 +626,64 @@ __device__ __forceinline__ Ray pixel_ray(const ViewDev &view, const MarchParams 
 
 // Opaque canvas: the ray ends at the world point of the canvas depth
 // (MapCanvasToRays: pixel (i, j) at depth d unprojected from NDC
-// (2i/W - 1, 2j/H - 1, 2d - 1); FP64, as in the oracle). FLT_MAX without a
-// canvas.
-__device__ __forceinline__ float canvas_ray_end(const ViewDev &view, const MarchParams &mp, int px,
-                                                int py)
+// (2i/W - 1, 2j/H - 1, 2d - 1); FP64, as in the oracle). FLT_MAX where the
+// pixel's end lies past `far`, the ray's furthest exit from a domain, so that
+// it cuts nothing off: an FP32 estimate less its own error bound (each term of
+// a row within 16 units in the last place of the sum of the row's magnitudes)
+// shows that for the background and for surfaces behind the volume. The FP64
+// pipe issues a warp in some 16 cycles, and the hundred or so FP64 operations
+// of the plain form for every pixel were more than half of a 1280 x 720 frame
+// (208 us; 140 us with the bound, 12 multiply-adds on matrices that hold the
+// NDC map, and one division).
+__device__ __noinline__ float canvas_ray_end(const ViewDev &view, const MarchParams &mp, int px, int py,
+                                             float far)
 {
-  float t_max = FLT_MAX;
-  if (mp.canvas_depth) {
-    const int64_t pix = (int64_t)py * mp.width + px;
-    const float din = mp.canvas_depth[pix];
-    const double xn = 2.0 * px / mp.width - 1.0, yn = 2.0 * py / mp.height - 1.0;
-    const double zn = 2.0 * (double)din - 1.0;
-    const double *I = view.inv_projview;
-    double P[4];
+  const float d = mp.canvas_depth[(int64_t)py * mp.width + px];
+  {
+    const float *U = view.unproject_f;
+    float P[4], E[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) P[q] = I[4 * q] * xn + I[4 * q + 1] * yn + I[4 * q + 2] * zn + I[4 * q + 3];
-    if (P[3] != 0.0) {
-      const double ex = P[0] / P[3] - view.origin[0], ey = P[1] / P[3] - view.origin[1],
-                   ez = P[2] / P[3] - view.origin[2];
-      t_max = (float)sqrt(ex * ex + ey * ey + ez * ez);
+    for (int q = 0; q < 4; ++q) {
+      const float a = U[4 * q] * (float)px, b = U[4 * q + 1] * (float)py, c = U[4 * q + 2] * d;
+      P[q] = a + b + c + U[4 * q + 3];
+      E[q] = 1e-6f * (fabsf(a) + fabsf(b) + fabsf(c) + fabsf(U[4 * q + 3]));
+    }
+    const float w = fabsf(P[3]);
+    if (w > 4.f * E[3]) {
+      float d2 = 0.f, err = 0.f;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const float x = P[a] / P[3];
+        const float e = x - view.origin[a];
+        d2 = fmaf(e, e, d2);
+        err += 1.5f * (E[a] + fabsf(x) * E[3]) / w + 1e-6f * fabsf(view.origin[a]);
+      }
+      if (sqrtf(d2) * 0.99999f - err > far) return FLT_MAX;
     }
   }
-  return t_max;
+  const double *U = view.unproject;
+  double P[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) P[q] = U[4 * q] * px + U[4 * q + 1] * py + U[4 * q + 2] * (double)d + U[4 * q + 3];
+  if (P[3] == 0.0) return FLT_MAX;
+  const double iw = 1.0 / P[3];
+  const double ex = P[0] * iw - view.origin[0], ey = P[1] * iw - view.origin[1],
+               ez = P[2] * iw - view.origin[2];
+  return (float)sqrt(ex * ex + ey * ey + ez * ez);
+}
+
+// Where the canvas ends a ray, for the domains of `mask`; FLT_MAX without a
+// canvas and where no domain is hit.
+__device__ __forceinline__ float ray_end(const DomainDev *doms, uint64_t mask, const Ray &r, const ViewDev &view,
+                                         const MarchParams &mp, int px, int py)
+{
+  if (!mp.canvas_depth) return FLT_MAX;
+  float far = -1.f;
+  for (uint64_t m = mask; m; m &= m - 1) {
+    float t0, t1;
+    if (slab(doms[__ffsll((long long)m) - 1], r, t0, t1)) far = fmaxf(far, t1);
+  }
+  return far < 0.f ? FLT_MAX : canvas_ray_end(view, mp, px, py, far);
 }
 
 // The pixel's final value from its composited partial (have = whether any
@@ -716,7 +752,7 @@ __device__ __forceinline__ void finish_pixel(const ViewDev &view, const MarchPar
 // and march_uniform's, operation for operation, so images are identical.
 constexpr int kUnifiedDomains = 16;
 
-template <int UNROLL, int SH>
+template <int UNROLL, int SH, int MODE>
 __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_t mask, const ViewDev &view,
                                                   const MarchParams &mp, const float4 *lut, int px, int py,
                                                   float4 &out, float &dep, float *g_state)
@@ -724,7 +760,7 @@ __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_
   int count = 0;
   const Ray r = pixel_ray(view, mp, px, py);
   float *st = g_state + threadIdx.x;
-  st[7 * kThreads] = canvas_ray_end(view, mp, px, py);
+  st[7 * kThreads] = MODE == kMarchUniform ? FLT_MAX : ray_end(doms, mask, r, view, mp, px, py);
   st[8 * kThreads] = __int_as_float(px);
   st[9 * kThreads] = __int_as_float(py);
   st[0 * kThreads] = 0.f;          // composited rgb
@@ -856,7 +892,8 @@ __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_
 
 // MODE: what the scene holds, and so which march code its kernel carries. The
 // calls of the rectilinear and cell-centred loops cost a 64-register kernel
-// some 90 bytes of spills, which one of uniform vertex fields does without.
+// some 90 bytes of spills, which one of uniform vertex fields does without;
+// that one has no canvas either (a canvas takes kMarchCells at least).
 template <int UNROLL, int MODE>
 __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, const ViewDev &view,
                                           const MarchParams &mp, const float4 *lut, int px, int py,
@@ -873,11 +910,11 @@ __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, 
       uni = uni && dm.kind == GVR_DOMAIN_UNIFORM && dm.assoc == GVR_ASSOC_VERTEX && dm.bshift == 3 &&
             !(mp.skip_empty && *dm.any_empty);
     }
-    if (uni) return render_ray_unified<UNROLL, 3>(doms, mask, view, mp, lut, px, py, out, dep, g_state);
+    if (uni) return render_ray_unified<UNROLL, 3, MODE>(doms, mask, view, mp, lut, px, py, out, dep, g_state);
   }
   int count = 0;
   const Ray r = pixel_ray(view, mp, px, py);
-  const float t_max = canvas_ray_end(view, mp, px, py);
+  const float t_max = MODE == kMarchUniform ? FLT_MAX : ray_end(doms, mask, r, view, mp, px, py);
 
   // Compositing state that lives across the march of a domain is parked in
   // shared memory (one word per thread per slot, st[k * kThreads]), so the
@@ -1184,7 +1221,8 @@ staged_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ V
   const int py = tile_y * kTile + (warp / PX) * PH + (lane / PW);
   const bool valid = px < mp.width && py < mp.height;
   const Ray r = pixel_ray(view, mp, valid ? px : 0, valid ? py : 0);
-  const float t_max = valid ? canvas_ray_end(view, mp, px, py) : FLT_MAX;
+  const float t_max =
+      valid ? ray_end(doms, mp.n_domains >= 64 ? ~0ull : (1ull << mp.n_domains) - 1ull, r, view, mp, px, py) : FLT_MAX;
   const float dt = mp.sample_dist;
   const float nm1 = (float)(mp.lut_size - 1);
 
@@ -1580,7 +1618,7 @@ layer_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
       const uint64_t all = mp.n_domains >= 64 ? ~0ull : ((1ull << mp.n_domains) - 1ull);
       float4 out;
       float dep;
-      count = render_ray<1, kMarchUniform>(doms, all, view, mp, lut, px, py, out, dep, s_state);
+      count = render_ray<1, kMarchCells>(doms, all, view, mp, lut, px, py, out, dep, s_state);
       const int64_t pix = (int64_t)py * mp.width + px;
       rgba[pix] = out;
       depth[pix] = dep;
@@ -1595,7 +1633,8 @@ layer_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
   }
 
   const Ray r = pixel_ray(view, mp, valid ? px : 0, valid ? py : 0);
-  const float t_max = valid ? canvas_ray_end(view, mp, px, py) : FLT_MAX;
+  const float t_max =
+      valid ? ray_end(doms, mp.n_domains >= 64 ? ~0ull : (1ull << mp.n_domains) - 1ull, r, view, mp, px, py) : FLT_MAX;
   const float dt = mp.sample_dist;
   const float nm1 = (float)(mp.lut_size - 1);
   float crgb[3] = {0.f, 0.f, 0.f}, ca = 0.f, cdepth = 0.f, covered = -FLT_MAX;
