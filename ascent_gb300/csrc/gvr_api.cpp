@@ -499,13 +499,12 @@ static int upload_field(gvr_scene *s, Domain &d, const void *field, int dtype, i
   if (d.dev.kind == GVR_DOMAIN_HEX) {
     const int rc = hex_update_field(d, field, dtype, stride, location);
     if (rc != GVR_OK) return rc;
-    s->table_dirty = true;
     s->classify_valid = false;
     return GVR_OK;
   }
   bool timed_out = false;
   if (d.dev.assoc == GVR_ASSOC_VERTEX) {
-    if (!s->d_flag && (e = cudaMalloc(&s->d_flag, sizeof(int))) != cudaSuccess)
+    if (!s->d_flag && (e = cudaMalloc(&s->d_flag, 4 * sizeof(int))) != cudaSuccess)
       return cuda_error(e, "cudaMalloc flag");
     e = launch_brick_field(field, dtype, stride, location == GVR_MEM_DEVICE, d.dev.dims, d.dev.bshift,
                            d.d_bricks, d.dev.nbrick, d.d_brick_range, d.range, d.stg, s->d_flag,
@@ -515,7 +514,6 @@ static int upload_field(gvr_scene *s, Domain &d, const void *field, int dtype, i
                            d.d_cells, d.range, d.stg, 0);
   }
   if (e != cudaSuccess) return cuda_error(e, "field upload");
-  s->table_dirty = true;
   s->classify_valid = false;
   if (timed_out) {
     // the bricks were rewritten with non-finite ranges: the domain's range
@@ -525,7 +523,6 @@ static int upload_field(gvr_scene *s, Domain &d, const void *field, int dtype, i
   }
   if (!(std::isfinite(d.range[0]) && std::isfinite(d.range[1])))
     return set_error(GVR_ERR_INVALID_ARGUMENT, "field contains non-finite values");
-  s->table_dirty = true;
   s->classify_valid = false;
   return GVR_OK;
 }
@@ -814,7 +811,6 @@ int gvr_scene_update_fields(gvr_scene *s, int n, const int *domain_ids, const vo
     e = launch_ranges_of_bricks(j, job_ranges.data(), job_bricks.data(), job_out.data(), st);
     if (e != cudaSuccess) return cuda_error(e, "field ranges");
   }
-  s->table_dirty = true;
   s->classify_valid = false;
   if (j > 0) {
     // ranges and the timeout flag in one copy
@@ -1029,13 +1025,22 @@ static int prepare_march(gvr_scene *s, const gvr_render_params *p, cudaStream_t 
     e = cudaMemcpyAsync(s->d_lut, p->lut_rgba, sizeof(float4) * p->lut_size, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->d_any_empty, 0, sizeof(int) * kMaxDomains, st);
     if (e != cudaSuccess) return cuda_error(e, "copy LUT");
+    const float2 *ranges[kMaxDomains];
+    int64_t n_bricks[kMaxDomains];
+    uint8_t *empty[kMaxDomains];
+    int *any[kMaxDomains];
+    int n = 0;
     for (size_t i = 0; i < s->domains.size(); ++i) {
-      Domain &d = s->domains[i];
+      const Domain &d = s->domains[i];
       if (d.dev.assoc != GVR_ASSOC_VERTEX) continue;
-      e = launch_empty_bricks(d.d_brick_range, d.n_bricks, s->d_lut, p->lut_size, p->lut_filter,
-                              mp.scalar_min, mp.inv_range, d.d_brick_empty, s->d_any_empty + i, st);
-      if (e != cudaSuccess) return cuda_error(e, "empty-brick pass");
+      ranges[n] = d.d_brick_range;
+      n_bricks[n] = d.n_bricks;
+      empty[n] = d.d_brick_empty;
+      any[n++] = s->d_any_empty + i;
     }
+    e = launch_empty_bricks(n, ranges, n_bricks, empty, any, s->d_lut, p->lut_size, p->lut_filter,
+                            mp.scalar_min, mp.inv_range, st);
+    if (e != cudaSuccess) return cuda_error(e, "empty-brick pass");
     s->classify_lut.assign(p->lut_rgba, p->lut_rgba + lut_floats);
     s->classify_filter = p->lut_filter;
     s->classify_smin = mp.scalar_min;

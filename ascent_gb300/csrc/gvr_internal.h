@@ -228,7 +228,7 @@ struct gvr_scene {
   float2 *d_ranges = nullptr;
   float2 *h_ranges = nullptr;
   int ranges_cap = 0;
-  int *d_flag = nullptr;  // timeout flag of single-field uploads
+  int *d_flag = nullptr;  // single-field uploads: timeout flag, unused, range (float2)
   cudaGraphExec_t batch_exec = nullptr;
   std::vector<unsigned char> batch_key;
   int batch_graph_builds = 0;
@@ -263,7 +263,8 @@ uint64_t launch_count();
 // ingest kernels (gvr_ingest.cu)
 // Brick a vertex field and read its range back (synchronises `stream`).
 // *d_timed_out is a device int the staged kernel sets when a bulk copy did
-// not complete within its bounded wait; *timed_out receives it.
+// not complete within its bounded wait (*timed_out receives it), the first of
+// four words: the range is reduced into the last two.
 cudaError_t launch_brick_field(const void *src, int dtype, int64_t stride,
                                int src_on_device, const int dims[3], int bshift,
                                float *d_bricks, const int nbrick[3],
@@ -291,11 +292,12 @@ cudaError_t launch_cells_field(const void *src, int dtype, int64_t stride,
                                int src_on_device, int64_t n, float *d_cells,
                                double range_out[2], Staging &stg,
                                cudaStream_t stream);
-cudaError_t launch_empty_bricks(const float2 *brick_range, int64_t n_bricks,
+// Classify the bricks of n domains' vertex fields against a transfer function
+// in one launch; *any_empty[j] becomes 1 when domain j has an empty brick.
+cudaError_t launch_empty_bricks(int n, const float2 *const *brick_range, const int64_t *n_bricks,
+                                uint8_t *const *brick_empty, int *const *any_empty,
                                 const float4 *d_lut, int lut_size, int lut_filter,
-                                float scalar_min, float inv_range,
-                                uint8_t *brick_empty, int *any_empty,
-                                cudaStream_t stream);
+                                float scalar_min, float inv_range, cudaStream_t stream);
 
 // sort / scan (gvr_sort.cu)
 size_t scan_scratch_words(int64_t n);
