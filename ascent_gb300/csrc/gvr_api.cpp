@@ -43,8 +43,92 @@ int cuda_error(cudaError_t e, const char *what)
 namespace {
 constexpr int kMaxPoolDevices = 64;
 std::mutex g_pool_mu;
-cudaMemPool_t g_pools[kMaxPoolDevices] = {};
+cudaMemPool_t g_pools[kMaxPoolDevices] = {};         // call scratch
+cudaMemPool_t g_scene_pools[kMaxPoolDevices] = {};   // scenes' memory
+cudaStream_t g_scene_streams[kMaxPoolDevices] = {};  // its allocations and frees
+
+// Free memory that a device's scene pool holds on to between scenes.
+constexpr uint64_t kScenePoolKeep = (uint64_t)4 << 30;
+
+// A pool of this library on `device` that keeps up to `keep` free bytes.
+cudaError_t make_pool(int device, uint64_t keep, cudaMemPool_t *out)
+{
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  cudaMemPool_t created = nullptr;
+  cudaError_t e = cudaMemPoolCreate(&created, &props);
+  if (e != cudaSuccess) return e;
+  if ((e = cudaMemPoolSetAttribute(created, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+    cudaMemPoolDestroy(created);
+    return e;
+  }
+  *out = created;
+  return cudaSuccess;
+}
 }  // namespace
+
+// Scenes' memory. An in-situ host makes a scene per publish, some 30 buffers
+// that cudaMalloc maps and cudaFree unmaps, each call a synchronisation: 3.9
+// of the 6.7 ms of a step with 1M new hexahedra, 1.2 of 3.4 ms of one with
+// four structured host domains. From a pool they cost a microsecond each; the
+// pool gives back what it holds beyond kScenePoolKeep at the next
+// synchronisation, all of it to gvr_scratch_trim, and when an allocation does
+// not fit. Allocations and frees are made on one stream of the pool's own on
+// which nothing runs, and an allocation is waited for, so that the memory may
+// be used on any stream and from any thread.
+cudaError_t device_alloc(void **ptr, size_t bytes)
+{
+  *ptr = nullptr;
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  if (device < 0 || device >= kMaxPoolDevices) return cudaMalloc(ptr, bytes);
+  cudaMemPool_t pool;
+  cudaStream_t stream;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (!g_scene_streams[device] &&
+        (e = cudaStreamCreateWithFlags(&g_scene_streams[device], cudaStreamNonBlocking)) != cudaSuccess)
+      return e;
+    if (!g_scene_pools[device] && (e = make_pool(device, kScenePoolKeep, &g_scene_pools[device])) != cudaSuccess)
+      return e;
+    pool = g_scene_pools[device];
+    stream = g_scene_streams[device];
+  }
+  e = cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
+  if (e == cudaErrorMemoryAllocation) {
+    // what the pools hold free may be what is missing
+    cudaGetLastError();
+    gvr_scratch_trim(device, 0, nullptr);
+    e = cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
+  }
+  return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
+}
+
+void device_free_idle(void *ptr)
+{
+  if (!ptr) return;
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxPoolDevices) {
+    cudaFree(ptr);
+    return;
+  }
+  cudaStream_t stream;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    stream = g_scene_streams[device];
+  }
+  cudaFreeAsync(ptr, stream);
+}
+
+void device_free(void *ptr)
+{
+  if (!ptr) return;
+  cudaDeviceSynchronize();
+  device_free_idle(ptr);
+}
 
 // The device's default memory pool gives its free memory back to the
 // system at every synchronisation (release threshold 0), so a call that
@@ -61,21 +145,7 @@ cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream)
   cudaMemPool_t pool;
   {
     std::lock_guard<std::mutex> lock(g_pool_mu);
-    if (!g_pools[device]) {
-      cudaMemPoolProps props{};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = device;
-      cudaMemPool_t created = nullptr;
-      if ((e = cudaMemPoolCreate(&created, &props)) != cudaSuccess) return e;
-      uint64_t keep = UINT64_MAX;
-      if ((e = cudaMemPoolSetAttribute(created, cudaMemPoolAttrReleaseThreshold, &keep)) !=
-          cudaSuccess) {
-        cudaMemPoolDestroy(created);
-        return e;
-      }
-      g_pools[device] = created;
-    }
+    if (!g_pools[device] && (e = make_pool(device, UINT64_MAX, &g_pools[device])) != cudaSuccess) return e;
     pool = g_pools[device];
   }
   return cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
@@ -87,12 +157,18 @@ int gvr_scratch_trim(int device, uint64_t keep_bytes, uint64_t *reserved_out)
 {
   using namespace gvr;
   if (device < 0) return set_error(GVR_ERR_INVALID_ARGUMENT, "negative device");
-  cudaMemPool_t pool = nullptr;
+  cudaMemPool_t pool = nullptr, scenes = nullptr;
   if (device < kMaxPoolDevices) {
     std::lock_guard<std::mutex> lock(g_pool_mu);
     pool = g_pools[device];
+    scenes = g_scene_pools[device];
   }
   uint64_t reserved = 0;
+  // what scenes that are gone have left in their pool; what scenes use stays
+  if (scenes) {
+    const cudaError_t e = cudaMemPoolTrimTo(scenes, (size_t)keep_bytes);
+    if (e != cudaSuccess) return cuda_error(e, "cudaMemPoolTrimTo");
+  }
   if (pool) {
     // blocks still in use are kept whatever keep_bytes says; memory freed
     // on a stream is returned once that free has completed
@@ -440,15 +516,16 @@ int gvr_scene_create(int device, gvr_scene **out)
   return GVR_OK;
 }
 
+// The caller has waited for the device.
 static void free_domain(Domain &d)
 {
-  cudaFree(d.d_bricks);
-  cudaFree(d.d_cells);
-  cudaFree(d.d_cell_rec);
-  cudaFree(d.d_brick_range);
-  cudaFree(d.d_brick_empty);
-  cudaFree(d.stg.buf);
-  cudaFree(d.stg.block_range);
+  device_free_idle(d.d_bricks);
+  device_free_idle(d.d_cells);
+  device_free_idle(d.d_cell_rec);
+  device_free_idle(d.d_brick_range);
+  device_free_idle(d.d_brick_empty);
+  device_free_idle(d.stg.buf);
+  device_free_idle(d.stg.block_range);
   free_hex(d);
   d = Domain();
 }
@@ -457,31 +534,32 @@ int gvr_scene_destroy(gvr_scene *s)
 {
   if (!s) return GVR_OK;
   cudaSetDevice(s->device);
+  cudaDeviceSynchronize();   // whatever still renders from the scene, on any stream
   for (Domain &d : s->domains) free_domain(d);
-  cudaFree(s->d_domains);
-  cudaFree(s->d_lut);
-  cudaFree(s->d_any_empty);
-  cudaFree(s->d_counters);
-  cudaFree(s->d_rgba_tmp);
-  cudaFree(s->d_depth_tmp);
-  cudaFree(s->d_views);
-  cudaFree(s->d_rects);
-  cudaFree(s->d_queue);
-  for (auto &t : s->tile_orders) cudaFree(t.second);
-  cudaFree(s->d_cost_order);
-  cudaFree(s->d_batch_rgba);
-  cudaFree(s->d_batch_depth);
+  device_free_idle(s->d_domains);
+  device_free_idle(s->d_lut);
+  device_free_idle(s->d_any_empty);
+  device_free_idle(s->d_counters);
+  device_free_idle(s->d_rgba_tmp);
+  device_free_idle(s->d_depth_tmp);
+  device_free_idle(s->d_views);
+  device_free_idle(s->d_rects);
+  device_free_idle(s->d_queue);
+  for (auto &t : s->tile_orders) device_free_idle(t.second);
+  device_free_idle(s->d_cost_order);
+  device_free_idle(s->d_batch_rgba);
+  device_free_idle(s->d_batch_depth);
   if (s->batch_exec) cudaGraphExecDestroy(s->batch_exec);
   if (s->own_stream) cudaStreamDestroy(s->own_stream);
   if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
   for (int b = 0; b < gvr_scene::kStageMax; ++b) {
-    cudaFree(s->stage[b]);
+    device_free_idle(s->stage[b]);
     if (s->copied[b]) cudaEventDestroy(s->copied[b]);
     if (s->consumed[b]) cudaEventDestroy(s->consumed[b]);
   }
-  cudaFree(s->d_ranges);
+  device_free_idle(s->d_ranges);
   cudaFreeHost(s->h_ranges);
-  cudaFree(s->d_flag);
+  device_free_idle(s->d_flag);
   delete s;
   return GVR_OK;
 }
@@ -504,8 +582,8 @@ static int upload_field(gvr_scene *s, Domain &d, const void *field, int dtype, i
   }
   bool timed_out = false;
   if (d.dev.assoc == GVR_ASSOC_VERTEX) {
-    if (!s->d_flag && (e = cudaMalloc(&s->d_flag, 4 * sizeof(int))) != cudaSuccess)
-      return cuda_error(e, "cudaMalloc flag");
+    if (!s->d_flag && (e = device_alloc((void **)&s->d_flag, 4 * sizeof(int))) != cudaSuccess)
+      return cuda_error(e, "allocate flag");
     e = launch_brick_field(field, dtype, stride, location == GVR_MEM_DEVICE, d.dev.dims, d.dev.bshift,
                            d.d_bricks, d.dev.nbrick, d.d_brick_range, d.range, d.stg, s->d_flag,
                            &timed_out, 0);
@@ -598,36 +676,37 @@ static int add_structured(gvr_scene *s, int kind, const int dims[3], const doubl
       d.bounds[2 * a] = d.dev.lo[a];
       d.bounds[2 * a + 1] = d.dev.hi[a];
     }
-    e = cudaMalloc(&d.d_cell_rec, sizeof(RectCell) * rec.size());
-    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc coords");
+    e = device_alloc((void **)&d.d_cell_rec, sizeof(RectCell) * rec.size());
+    if (e != cudaSuccess) return cuda_error(e, "allocate coords");
     e = cudaMemcpy(d.d_cell_rec, rec.data(), sizeof(RectCell) * rec.size(), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) { free_domain(d); return cuda_error(e, "copy coords"); }
+    if (e != cudaSuccess) { cudaDeviceSynchronize(); free_domain(d); return cuda_error(e, "copy coords"); }
     d.dev.cell_rec = d.d_cell_rec;
   }
   if (assoc == GVR_ASSOC_VERTEX) {
     d.n_values = (size_t)dims[0] * dims[1] * dims[2];
     d.n_bricks = (int64_t)d.dev.nbrick[0] * d.dev.nbrick[1] * d.dev.nbrick[2];
     if (d.n_bricks * brick_floats(d.dev.bshift) >= (int64_t)1 << 31) {
+      cudaDeviceSynchronize();
       free_domain(d);
       return set_error(GVR_ERR_UNSUPPORTED,
                        "a domain's bricked field must hold < 2^31 floats (about 1290^3 nodes); "
                        "split it into more domains");
     }
-    e = cudaMalloc(&d.d_bricks, sizeof(float) * brick_floats(d.dev.bshift) * d.n_bricks);
-    if (e == cudaSuccess) e = cudaMalloc(&d.d_brick_range, sizeof(float2) * d.n_bricks);
-    if (e == cudaSuccess) e = cudaMalloc(&d.d_brick_empty, d.n_bricks);
+    e = device_alloc((void **)&d.d_bricks, sizeof(float) * brick_floats(d.dev.bshift) * d.n_bricks);
+    if (e == cudaSuccess) e = device_alloc((void **)&d.d_brick_range, sizeof(float2) * d.n_bricks);
+    if (e == cudaSuccess) e = device_alloc((void **)&d.d_brick_empty, d.n_bricks);
     if (e == cudaSuccess) e = cudaMemset(d.d_brick_empty, 0, d.n_bricks);
   } else {
     d.n_values = (size_t)(dims[0] - 1) * (dims[1] - 1) * (dims[2] - 1);
-    e = cudaMalloc(&d.d_cells, sizeof(float) * d.n_values);
+    e = device_alloc((void **)&d.d_cells, sizeof(float) * d.n_values);
   }
-  if (e != cudaSuccess) { free_domain(d); return cuda_error(e, "cudaMalloc field"); }
+  if (e != cudaSuccess) { cudaDeviceSynchronize(); free_domain(d); return cuda_error(e, "allocate field"); }
   d.dev.bricks = d.d_bricks;
   d.dev.cells = d.d_cells;
   d.dev.brick_range = d.d_brick_range;
   d.dev.brick_empty = d.d_brick_empty;
   int rc = upload_field(s, d, field, dtype, stride, location);
-  if (rc != GVR_OK) { free_domain(d); return rc; }
+  if (rc != GVR_OK) { cudaDeviceSynchronize(); free_domain(d); return rc; }
   s->domains.push_back(d);
   s->table_dirty = true;
   if (domain_id) *domain_id = (int)s->domains.size() - 1;
@@ -692,13 +771,13 @@ int gvr_scene_update_fields(gvr_scene *s, int n, const int *domain_ids, const vo
     return (size_t)((int64_t)(d.n_values - 1) * stride + 1) * esz;
   };
   if (n > s->ranges_cap) {
-    cudaFree(s->d_ranges);
+    device_free(s->d_ranges);
     cudaFreeHost(s->h_ranges);
     s->d_ranges = nullptr;
     s->h_ranges = nullptr;
     s->ranges_cap = 0;
-    if ((e = cudaMalloc(&s->d_ranges, sizeof(float2) * (n + 1))) != cudaSuccess)
-      return cuda_error(e, "cudaMalloc ranges");
+    if ((e = device_alloc((void **)&s->d_ranges, sizeof(float2) * (n + 1))) != cudaSuccess)
+      return cuda_error(e, "allocate ranges");
     if ((e = cudaMallocHost(&s->h_ranges, sizeof(float2) * (n + 1))) != cudaSuccess)
       return cuda_error(e, "cudaMallocHost ranges");
     s->ranges_cap = n;
@@ -734,14 +813,14 @@ int gvr_scene_update_fields(gvr_scene *s, int n, const int *domain_ids, const vo
       // the old buffers may still be read by bricking from an earlier call
       if ((e = cudaDeviceSynchronize()) != cudaSuccess) return cuda_error(e, "staging");
       for (int b = 0; b < gvr_scene::kStageMax; ++b) {
-        cudaFree(s->stage[b]);
+        device_free(s->stage[b]);
         s->stage[b] = nullptr;
       }
       const size_t bytes = std::max(need, s->stage_bytes);
       s->stage_bytes = 0;
       s->stage_count = 0;
       for (int b = 0; b < want; ++b)
-        if ((e = cudaMalloc(&s->stage[b], bytes)) != cudaSuccess) return cuda_error(e, "staging");
+        if ((e = device_alloc((void **)&s->stage[b], bytes)) != cudaSuccess) return cuda_error(e, "staging");
       s->stage_bytes = bytes;
       s->stage_count = want;
     }
@@ -943,16 +1022,16 @@ static int ensure_buffers(gvr_scene *s, int64_t pixels, int lut_size)
   cudaError_t e;
   if (s->table_dirty || s->d_domains_cap < (int)s->domains.size()) {
     if (s->d_domains_cap < (int)s->domains.size()) {
-      cudaFree(s->d_domains);
+      device_free(s->d_domains);
       s->d_domains = nullptr;
-      e = cudaMalloc(&s->d_domains, sizeof(DomainDev) * kMaxDomains);
-      if (e != cudaSuccess) return cuda_error(e, "cudaMalloc domain table");
+      e = device_alloc((void **)&s->d_domains, sizeof(DomainDev) * kMaxDomains);
+      if (e != cudaSuccess) return cuda_error(e, "allocate domain table");
       s->d_domains_cap = kMaxDomains;
     }
     if (!s->d_any_empty) {
-      e = cudaMalloc(&s->d_any_empty, sizeof(int) * kMaxDomains);
+      e = device_alloc((void **)&s->d_any_empty, sizeof(int) * kMaxDomains);
       if (e == cudaSuccess) e = cudaMemset(s->d_any_empty, 0, sizeof(int) * kMaxDomains);
-      if (e != cudaSuccess) return cuda_error(e, "cudaMalloc empty flags");
+      if (e != cudaSuccess) return cuda_error(e, "allocate empty flags");
     }
     std::vector<DomainDev> h(s->domains.size());
     for (size_t i = 0; i < h.size(); ++i) {
@@ -966,23 +1045,23 @@ static int ensure_buffers(gvr_scene *s, int64_t pixels, int lut_size)
     s->table_dirty = false;
   }
   if (!s->d_lut) {
-    e = cudaMalloc(&s->d_lut, sizeof(float4) * kMaxLut);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc LUT");
+    e = device_alloc((void **)&s->d_lut, sizeof(float4) * kMaxLut);
+    if (e != cudaSuccess) return cuda_error(e, "allocate LUT");
   }
   if (!s->d_counters) {
-    e = cudaMalloc(&s->d_counters, sizeof(unsigned long long) * 4);
+    e = device_alloc((void **)&s->d_counters, sizeof(unsigned long long) * 4);
     if (e == cudaSuccess) e = cudaMemset(s->d_counters, 0, sizeof(unsigned long long) * 4);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc counters");
+    if (e != cudaSuccess) return cuda_error(e, "allocate counters");
   }
   if (pixels > s->tmp_pixels) {
-    cudaFree(s->d_rgba_tmp);
-    cudaFree(s->d_depth_tmp);
+    device_free(s->d_rgba_tmp);
+    device_free(s->d_depth_tmp);
     s->d_rgba_tmp = nullptr;
     s->d_depth_tmp = nullptr;
     s->tmp_pixels = 0;
-    e = cudaMalloc(&s->d_rgba_tmp, sizeof(float4) * pixels);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_depth_tmp, sizeof(float) * pixels);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc image");
+    e = device_alloc((void **)&s->d_rgba_tmp, sizeof(float4) * pixels);
+    if (e == cudaSuccess) e = device_alloc((void **)&s->d_depth_tmp, sizeof(float) * pixels);
+    if (e != cudaSuccess) return cuda_error(e, "allocate image");
     s->tmp_pixels = pixels;
   }
   (void)lut_size;
@@ -1100,11 +1179,11 @@ static int tile_order(gvr_scene *s, int W, int H, const int **out)
   for (int y = 0; y < ty; ++y)
     for (int x = 0; x < tx; ++x) ord[cnt[key(x, y)]++] = y * tx + x;
   int *d = nullptr;
-  cudaError_t e = cudaMalloc(&d, sizeof(int) * n);
-  if (e != cudaSuccess) return cuda_error(e, "cudaMalloc tile order");
+  cudaError_t e = device_alloc((void **)&d, sizeof(int) * n);
+  if (e != cudaSuccess) return cuda_error(e, "allocate tile order");
   e = cudaMemcpy(d, ord.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
-    cudaFree(d);
+    device_free(d);
     return cuda_error(e, "copy tile order");
   }
   s->tile_orders[{tx, ty}] = d;
@@ -1272,12 +1351,12 @@ static int render_one(gvr_scene *s, const gvr_camera *camera, const gvr_render_p
       // sort launch)
       if (s->d_cost_order && (e = cudaStreamSynchronize(st)) != cudaSuccess)
         return cuda_error(e, "tile cost order");
-      cudaFree(s->d_cost_order);
+      device_free(s->d_cost_order);
       s->d_cost_order = nullptr;
       s->cost_order_cap = 0;
-      e = cudaMalloc(&s->d_cost_order, sizeof(int) * (2 * n_tiles + 1));
+      e = device_alloc((void **)&s->d_cost_order, sizeof(int) * (2 * n_tiles + 1));
       if (e == cudaSuccess) e = cudaMemsetAsync(s->d_cost_order + 2 * n_tiles, 0, sizeof(int), st);
-      if (e != cudaSuccess) return cuda_error(e, "cudaMalloc tile cost order");
+      if (e != cudaSuccess) return cuda_error(e, "allocate tile cost order");
       s->cost_order_cap = n_tiles;
     }
     e = launch_tile_cost_order(s->d_domains, view, mp, s->d_cost_order,
@@ -1376,32 +1455,32 @@ int gvr_render_volume_batch(gvr_scene *s, const gvr_camera *cameras, int n_views
   }
   const int nd = (int)s->domains.size();
   if (n_views > s->views_cap) {
-    cudaFree(s->d_views);
+    device_free(s->d_views);
     s->d_views = nullptr;
     s->views_cap = 0;
-    if ((e = cudaMalloc(&s->d_views, sizeof(ViewDev) * n_views)) != cudaSuccess)
-      return cuda_error(e, "cudaMalloc views");
+    if ((e = device_alloc((void **)&s->d_views, sizeof(ViewDev) * n_views)) != cudaSuccess)
+      return cuda_error(e, "allocate views");
     s->views_cap = n_views;
   }
   if (n_views * nd > s->rects_cap) {
-    cudaFree(s->d_rects);
+    device_free(s->d_rects);
     s->d_rects = nullptr;
     s->rects_cap = 0;
-    if ((e = cudaMalloc(&s->d_rects, sizeof(int4) * n_views * nd)) != cudaSuccess)
-      return cuda_error(e, "cudaMalloc rects");
+    if ((e = device_alloc((void **)&s->d_rects, sizeof(int4) * n_views * nd)) != cudaSuccess)
+      return cuda_error(e, "allocate rects");
     s->rects_cap = n_views * nd;
   }
-  if (!s->d_queue && (e = cudaMalloc(&s->d_queue, 256)) != cudaSuccess)
-    return cuda_error(e, "cudaMalloc queue");
+  if (!s->d_queue && (e = device_alloc((void **)&s->d_queue, 256)) != cudaSuccess)
+    return cuda_error(e, "allocate queue");
   if (out_location == GVR_MEM_HOST && pixels * n_views > s->batch_pixels) {
-    cudaFree(s->d_batch_rgba);
-    cudaFree(s->d_batch_depth);
+    device_free(s->d_batch_rgba);
+    device_free(s->d_batch_depth);
     s->d_batch_rgba = nullptr;
     s->d_batch_depth = nullptr;
     s->batch_pixels = 0;
-    e = cudaMalloc(&s->d_batch_rgba, sizeof(float4) * pixels * n_views);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_batch_depth, sizeof(float) * pixels * n_views);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc batch images");
+    e = device_alloc((void **)&s->d_batch_rgba, sizeof(float4) * pixels * n_views);
+    if (e == cudaSuccess) e = device_alloc((void **)&s->d_batch_depth, sizeof(float) * pixels * n_views);
+    if (e != cudaSuccess) return cuda_error(e, "allocate batch images");
     s->batch_pixels = pixels * n_views;
   }
   MarchParams mp;

@@ -424,7 +424,7 @@ int grid_for(int64_t n, int threads = 256)
 template <typename T>
 cudaError_t dev_alloc(T **p, size_t count)
 {
-  return cudaMalloc((void **)p, sizeof(T) * std::max<size_t>(count, 1));
+  return device_alloc((void **)p, sizeof(T) * std::max<size_t>(count, 1));
 }
 
 // Stage `bytes` of a host array on the device (or return the device pointer).
@@ -435,7 +435,7 @@ cudaError_t stage(const void *src, size_t bytes, int on_device, void **owned, co
     *out = src;
     return cudaSuccess;
   }
-  cudaError_t e = cudaMalloc(owned, bytes);
+  cudaError_t e = device_alloc(owned, bytes);
   if (e == cudaSuccess) e = cudaMemcpy(*owned, src, bytes, cudaMemcpyHostToDevice);
   *out = *owned;
   return e;
@@ -443,20 +443,21 @@ cudaError_t stage(const void *src, size_t bytes, int on_device, void **owned, co
 
 }  // namespace
 
+// The caller has waited for the device.
 void free_hex(Domain &d)
 {
-  cudaFree(d.d_nodes);
-  cudaFree(d.d_conn);
-  cudaFree(d.d_bvh);
-  cudaFree(d.d_codes);
-  cudaFree(d.d_ids);
-  cudaFree(d.d_left);
-  cudaFree(d.d_right);
-  cudaFree(d.d_parent);
-  cudaFree(d.d_inner_box);
-  cudaFree(d.d_nbr);
+  device_free_idle(d.d_nodes);
+  device_free_idle(d.d_conn);
+  device_free_idle(d.d_bvh);
+  device_free_idle(d.d_codes);
+  device_free_idle(d.d_ids);
+  device_free_idle(d.d_left);
+  device_free_idle(d.d_right);
+  device_free_idle(d.d_parent);
+  device_free_idle(d.d_inner_box);
+  device_free_idle(d.d_nbr);
   d.d_nbr = nullptr;
-  cudaFree(d.d_coef);
+  device_free_idle(d.d_coef);
   d.d_coef = nullptr;
   d.d_nodes = nullptr;
   d.d_conn = nullptr;
@@ -478,7 +479,7 @@ static int node_range(Domain &d)
     count_launch();
     e = cudaMemcpy(h.data(), part, sizeof(float2) * gb, cudaMemcpyDeviceToHost);
   }
-  cudaFree(part);
+  device_free(part);
   if (e != cudaSuccess) return cuda_error(e, "hex field range");
   double lo = INFINITY, hi = -INFINITY;
   for (const float2 &r : h) {
@@ -506,10 +507,10 @@ int hex_update_field(Domain &d, const void *field, int dtype, int64_t stride, in
   cudaError_t e = cudaSuccess;
   if (location != GVR_MEM_DEVICE) {
     if (bytes > d.stg.bytes) {
-      cudaFree(d.stg.buf);
+      device_free(d.stg.buf);
       d.stg.buf = nullptr;
       d.stg.bytes = 0;
-      e = cudaMalloc(&d.stg.buf, bytes);
+      e = device_alloc((void **)&d.stg.buf, bytes);
       if (e != cudaSuccess) return cuda_error(e, "hex field staging");
       d.stg.bytes = bytes;
     }
@@ -525,7 +526,7 @@ int hex_update_field(Domain &d, const void *field, int dtype, int64_t stride, in
     count_launch();
     e = cudaMemcpy(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost);
   }
-  cudaFree(flag);
+  device_free(flag);
   if (e != cudaSuccess) return cuda_error(e, "hex field update");
   if (bad) return set_error(GVR_ERR_INVALID_ARGUMENT, "field contains non-finite values");
   coef_kernel<<<grid_for(d.n_cells), 256>>>(d.d_nodes, d.d_conn, d.n_cells, d.d_coef);
@@ -561,8 +562,8 @@ static int build_neighbours(Domain &d)
   face_key_kernel<<<grid_for(nf), 256>>>(d.d_conn, nf, key, face);
   count_launch();
   NB_TRY(radix_sort_pairs<uint32_t>(key, face, key_tmp, face_tmp, nf, bits, scr, 0), "sort faces");
-  cudaFree(key);
-  cudaFree(key_tmp);
+  device_free(key);
+  device_free(key_tmp);
   key = key_tmp = nullptr;
   NB_TRY(dev_alloc(&key2, nf), "alloc face keys");
   NB_TRY(dev_alloc(&key2_tmp, nf), "alloc face keys");
@@ -576,13 +577,13 @@ static int build_neighbours(Domain &d)
   NB_TRY(cudaDeviceSynchronize(), "neighbours");
 done:
 #undef NB_TRY
-  cudaFree(key);
-  cudaFree(key_tmp);
-  cudaFree(key2);
-  cudaFree(key2_tmp);
-  cudaFree(face);
-  cudaFree(face_tmp);
-  cudaFree(scr);
+  device_free(key);
+  device_free(key_tmp);
+  device_free(key2);
+  device_free(key2_tmp);
+  device_free(face);
+  device_free(face_tmp);
+  device_free(scr);
   d.nbr_build_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
   return rc;
 }
@@ -704,15 +705,16 @@ static int build_hex(Domain &d, const void *x, const void *y, const void *z, int
   }
 done:
 #undef HEX_TRY
-  for (void *p : own) cudaFree(p);
-  cudaFree(d_flag);
-  cudaFree(leaf_lo);
-  cudaFree(leaf_hi);
-  cudaFree(part);
-  cudaFree(keys_tmp);
-  cudaFree(vals_tmp);
-  cudaFree(sort_scr);
-  cudaFree(counters);
+  if (rc != GVR_OK) cudaDeviceSynchronize();   // otherwise the tree was waited for
+  for (void *p : own) device_free_idle(p);
+  device_free_idle(d_flag);
+  device_free_idle(leaf_lo);
+  device_free_idle(leaf_hi);
+  device_free_idle(part);
+  device_free_idle(keys_tmp);
+  device_free_idle(vals_tmp);
+  device_free_idle(sort_scr);
+  device_free_idle(counters);
   d.bvh_build_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
   if (rc == GVR_OK) rc = build_neighbours(d);
   d.dev.hex_nbr = d.d_nbr;
@@ -763,10 +765,11 @@ int gvr_scene_add_hex(gvr_scene *s, int64_t n_nodes, const void *x, const void *
   int rc = build_hex(d, x, y, z, coord_dtype, conn, conn_int64 ? 1 : 0, field, dtype, association,
                      location);
   if (rc != GVR_OK) {
+    cudaDeviceSynchronize();
     free_hex(d);
-    cudaFree(d.d_cells);
-    cudaFree(d.stg.buf);
-    cudaFree(d.stg.block_range);
+    device_free(d.d_cells);
+    device_free(d.stg.buf);
+    device_free(d.stg.block_range);
     return rc;
   }
   s->domains.push_back(d);
@@ -835,9 +838,9 @@ int gvr_scene_hex_locate(gvr_scene *s, int domain_id, const float *points, int n
   cudaError_t e = cudaSetDevice(s->device);
   float *dp = nullptr, *dr = nullptr;
   int *dc = nullptr;
-  if (e == cudaSuccess) e = cudaMalloc(&dp, sizeof(float) * 3 * n);
-  if (e == cudaSuccess) e = cudaMalloc(&dr, sizeof(float) * 3 * n);
-  if (e == cudaSuccess) e = cudaMalloc(&dc, sizeof(int) * n);
+  if (e == cudaSuccess) e = device_alloc((void **)&dp, sizeof(float) * 3 * n);
+  if (e == cudaSuccess) e = device_alloc((void **)&dr, sizeof(float) * 3 * n);
+  if (e == cudaSuccess) e = device_alloc((void **)&dc, sizeof(int) * n);
   if (e == cudaSuccess) e = cudaMemcpy(dp, points, sizeof(float) * 3 * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
     locate_kernel<<<grid_for(n), 256>>>(d.dev, dp, n, dc, dr);
@@ -846,9 +849,9 @@ int gvr_scene_hex_locate(gvr_scene *s, int domain_id, const float *points, int n
   }
   if (e == cudaSuccess) e = cudaMemcpy(cells, dc, sizeof(int) * n, cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(rst, dr, sizeof(float) * 3 * n, cudaMemcpyDeviceToHost);
-  cudaFree(dp);
-  cudaFree(dr);
-  cudaFree(dc);
+  device_free(dp);
+  device_free(dr);
+  device_free(dc);
   if (e != cudaSuccess) return cuda_error(e, "hex locate");
   return GVR_OK;
 }

@@ -459,10 +459,10 @@ cudaError_t stage_source(const void *src, int dtype, int64_t stride,
   const size_t esz = dtype == GVR_DTYPE_FLOAT64 ? 8 : 4;
   const size_t bytes = (size_t)((n - 1) * stride + 1) * esz;
   if (bytes > stg.bytes) {
-    cudaFree(stg.buf);
+    device_free(stg.buf);
     stg.buf = nullptr;
     stg.bytes = 0;
-    cudaError_t e = cudaMalloc(&stg.buf, bytes);
+    cudaError_t e = device_alloc((void **)&stg.buf, bytes);
     if (e != cudaSuccess) return e;
     stg.bytes = bytes;
   }
@@ -621,7 +621,7 @@ cudaError_t launch_cells_field(const void *src, int dtype, int64_t stride,
   int blocks = (int)((n + 255) / 256);
   if (blocks > 4096) blocks = 4096;
   if (!stg.block_range) {
-    e = cudaMalloc(&stg.block_range, sizeof(float2) * 4096);
+    e = device_alloc((void **)&stg.block_range, sizeof(float2) * 4096);
     if (e != cudaSuccess) return e;
   }
   float2 *d_br = stg.block_range;

@@ -256,6 +256,13 @@ void make_view(const gvr_camera &cam, int width, int height, ViewDev *v);
 // cudaFreeAsync
 cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
 
+// Device memory of scenes and of their builds, from a second pool of this
+// library: usable at once on any stream. device_free waits for the device
+// first, as cudaFree does; device_free_idle is for a caller that has.
+cudaError_t device_alloc(void **ptr, size_t bytes);
+void device_free(void *ptr);
+void device_free_idle(void *ptr);
+
 // kernels launched by this library since it was loaded
 void count_launch(int n = 1);
 uint64_t launch_count();
