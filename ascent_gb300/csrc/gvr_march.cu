@@ -94,6 +94,14 @@ struct Partial {
   int count;    // samples the stepping rule took
 };
 
+// The colour of a saturated scalar, the filter known at compile time: a branch
+// per sample on a uniform value costs four instructions of some ninety.
+template <bool LIN>
+__device__ __forceinline__ float4 lut_color(const float4 *lut, const MarchParams &mp, float nm1, float s)
+{
+  return LIN ? lut_fetch(lut, mp.lut_size, GVR_LUT_LINEAR, s) : lut_nearest(lut, nm1, s);
+}
+
 // a / b from y = RN(1 / b): the product a y corrected by its residual
 // (Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000", 1990). Three operations against the eight or so and the
@@ -326,8 +334,8 @@ __device__ __noinline__ Partial march_cells(const DomainDev &dm, const Ray r, fl
 // 8 corners are loaded from the bricks unless the sample before was in the
 // same cell (lc, last_off hold that cell's), and v[u] is the trilinear
 // value. ok[u]: the sample lies before t1 (and, with LIMIT, its index
-// before kend); a sample that does not is placed at t0 so that its loads
-// stay inside the domain. Shared by the per-domain loops and the one-loop
+// before kend); the cell of one that does not is clamped to the domain like any
+// other's, so its loads stay inside. Shared by the per-domain loops and the one-loop
 // domain walk, so all of them take the same samples with the same
 // arithmetic.
 template <int UNROLL, int SH, bool LIMIT>
@@ -338,21 +346,23 @@ __device__ __forceinline__ void sample_cells(const float *__restrict__ bricks, c
                                              bool ok[UNROLL])
 {
   constexpr int BC = brick_cells(SH), BN = brick_nodes(SH), BF = brick_floats(SH);
+  const float kf = (float)k;
 #pragma unroll
   for (int u = 0; u < UNROLL; ++u) {
-    float t = fmaf((float)(k + u), dt, t0);
+    const float t = fmaf(kf + (float)u, dt, t0);
     ok[u] = LIMIT ? (k + u < kend && t < t1) : t < t1;
-    t = ok[u] ? t : t0;
+    // brick c >> SH, place c - (c >> SH) * BC in it: the offset is linear in
+    // both, so the place needs no operation of its own
     int off = 0;
     float w[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const float g = fmaf(t, B[a], A[a]);
-      const int c = max(0, min((int)g, cmax[a]));
+      const int c = __vimin_s32_relu((int)g, cmax[a]);   // max(0, min)
       w[a] = g - (float)c;
-      const int hi = c >> SH, lo = c & (BC - 1);
-      off += a == 0 ? hi * BF + lo
-                    : (a == 1 ? hi * sy + lo * BN : hi * sz + lo * BN * BN);
+      const int hi = c >> SH;
+      off += a == 0 ? hi * (BF - BC) + c
+                    : (a == 1 ? hi * (sy - BC * BN) + c * BN : hi * (sz - BC * BN * BN) + c * (BN * BN));
     }
     if (off != last_off) {
       const float *p = bricks + off;
@@ -380,7 +390,7 @@ __device__ __forceinline__ void sample_cells(const float *__restrict__ bricks, c
 // before it reuses that cell's corners from registers (the same values, so
 // the result does not change). Blending stays sequential and stops exactly
 // where the one-sample loop stops.
-template <int UNROLL, int SH>
+template <int UNROLL, int SH, bool LIN>
 __device__ __forceinline__ int march_uniform(const DomainDev &dm, const Ray &r, float t0,
                                              float t1, const MarchParams &mp,
                                              const float4 *lut, float thr, float4 &acc)
@@ -412,12 +422,7 @@ __device__ __forceinline__ int march_uniform(const DomainDev &dm, const Ray &r, 
     for (int u = 0; u < UNROLL; ++u) {
       if (!ok[u]) return k + u;
       const float s = __saturatef((v[u] - mp.scalar_min) * mp.inv_range);
-      float4 col;
-      if (mp.lut_filter == GVR_LUT_LINEAR) {
-        col = lut_fetch(lut, mp.lut_size, GVR_LUT_LINEAR, s);
-      } else {
-        col = lut_nearest(lut, nm1, s);
-      }
+      const float4 col = lut_color<LIN>(lut, mp, nm1, s);
       const float wa = (1.f - acc.w) * col.w;
       acc.x = fmaf(wa, col.x, acc.x);
       acc.y = fmaf(wa, col.y, acc.y);
@@ -758,24 +763,42 @@ __device__ __forceinline__ void finish_pixel(const ViewDev &view, const MarchPar
   }
 }
 
-// render_ray for scenes whose domains (at most kUnifiedDomains) are all
-// uniform vertex fields with no empty bricks to jump, bricked alike: one
-// loop walks the samples of every domain the ray crosses. A lane that
-// reaches the end of a domain (or its opacity threshold) blends that
+// render_ray for rays whose domains are all uniform vertex fields in 8^3-cell
+// bricks: one loop walks the samples of every domain the ray crosses. A lane
+// that reaches the end of a domain (or its opacity threshold) blends that
 // domain's partial and sets up the next domain inside the same loop, while
 // the other lanes of its warp go on sampling; in the per-domain form a
 // lane that left its domain first waits at the end of the domain's loop
-// until the last lane of the warp leaves it. The domain order, the sample
-// positions, the per-domain accumulation and the blend are render_ray's
-// and march_uniform's, operation for operation, so images are identical.
-constexpr int kUnifiedDomains = 16;
+// until the last lane of the warp leaves it. Empty bricks are met in the same
+// loop too: after a group of samples a lane whose last sample lies in another
+// brick than before looks that brick up, and where it is empty passes over
+// its samples (and the next bricks' while they are empty), again without the
+// other lanes; only the bricks' own loop would make them wait at each brick.
+// No lane leaves a group early: a lane that is done takes samples of weight
+// zero until all lanes of the warp are done, so that the warp stays together.
+// The domain order, the sample positions, the per-domain accumulation and the
+// blend are render_ray's and march_uniform's, operation for operation, so
+// images are identical.
+//
+// Bound by instructions and, at a sample per half cell and pixel, as much by
+// L1 wavefronts (75% of their peak, 33 a sample of a warp). 64 views at 512^2
+// of 37 domains, whose rays cross some six of them: a loop per domain and per
+// brick kept 18.4 of 32 lanes active and took 36.6 ms; this one keeps 26.3 and
+// takes 24.1. The 513^3 field in 8 domains at 1024^2: 1468 us with branches
+// out of the group's samples, 1433 us so.
+// Steps of so many cells and more pass over no bricks: each holds four samples
+// at most (a frame of the 513^3 field at 100 samples, 5 cells a step, with its
+// publish: 534 us with, 475 us without; at a half cell a step the two are
+// within 2%).
+constexpr float kSkipCells = 2.f;
+constexpr int kWalkDomains = 10;   // domains of a ray ordered at a time, 6 bits each in two words
 
-template <int UNROLL, int SH, int MODE>
+template <int UNROLL, int MODE, bool LIN>
 __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_t mask, const ViewDev &view,
                                                   const MarchParams &mp, const float4 *lut, int px, int py,
-                                                  float4 &out, float &dep, float *g_state)
+                                                  float4 &out, float &dep, float *g_state, bool any_hidden)
 {
-  int count = 0;
+  constexpr int BF = brick_floats(3);
   const Ray r = pixel_ray(view, mp, px, py);
   float *st = g_state + threadIdx.x;
   st[7 * kThreads] = MODE == kMarchUniform ? FLT_MAX : ray_end(doms, mask, r, view, mp, px, py);
@@ -787,53 +810,31 @@ __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_
   st[3 * kThreads] = 0.f;          // depth of the front partial
   st[5 * kThreads] = -FLT_MAX;     // furthest exit covered
   // the ray's domains in render_ray's order, (entry distance, index)
-  // ascending, 4 bits each; kept in two state slots with the next position
-  {
-    uint64_t seq = 0;
-    int nseq = 0;
-    float last_t0 = -FLT_MAX;
-    int last_d = -1;
-    for (;;) {
-      int best = -1;
-      float bt0 = FLT_MAX;
-      for (uint64_t m = mask; m; m &= m - 1) {
-        const int dd = __ffsll((long long)m) - 1;
-        float t0, t1;
-        if (!slab(doms[dd], r, t0, t1)) continue;
-        const bool after = t0 > last_t0 || (t0 == last_t0 && dd > last_d);
-        const bool before = best < 0 || t0 < bt0;
-        if (after && before) { best = dd; bt0 = t0; }
-      }
-      if (best < 0) break;
-      seq |= (uint64_t)best << (4 * nseq);
-      ++nseq;
-      last_t0 = bt0;
-      last_d = best;
-    }
-    st[4 * kThreads] = __int_as_float((int)(uint32_t)seq);
-    st[6 * kThreads] = __int_as_float((int)(uint32_t)(seq >> 32));
-    st[5 * kThreads] = -FLT_MAX;
-    // next position in the sequence (low 8 bits) and its length (next 8)
-    st[10 * kThreads] = __int_as_float(nseq << 8);
-  }
+  // ascending, kWalkDomains at a time: five in each of slots 4 and 6, and in
+  // slot 10 the next position, their number << 8, the last of them << 16, and
+  // bit 24: there are more
+  st[10 * kThreads] = __int_as_float(0xff << 16 | 1 << 24);
   float ca = 0.f;
   bool have = false;
-  bool fresh = true;      // the next iteration starts a domain
+  bool live = true;       // the ray has samples left
+  bool fresh = true;      // the next turn starts a domain
   bool started = false;   // a domain has been marched (its partial is pending)
+  const unsigned warp = __activemask();
   const float dt = mp.sample_dist;
   const float nm1 = (float)(mp.lut_size - 1);
-  constexpr int BC = brick_cells(SH), BN = brick_nodes(SH), BF = brick_floats(SH);
   float A[3] = {0.f, 0.f, 0.f}, B[3] = {0.f, 0.f, 0.f};
   int cmax[3] = {0, 0, 0};
   int sy = 0, sz = 0;
   const float *__restrict__ bricks = nullptr;
+  int hidden = -1;        // the domain if it has empty bricks, else -1
   float bt0 = 0.f, bt1 = 0.f, thr = 2.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  int k = 0;
-  int last_off = -1;
+  int k = 0, count = 0;
+  int last_off = 0, brick = -1;
   float lc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (;;) {
     if (fresh) {
+      fresh = false;
       if (started && !(acc.w < mp.alpha_cull)) {
         if (!have) {
           st[0 * kThreads] = acc.x; st[1 * kThreads] = acc.y; st[2 * kThreads] = acc.z;
@@ -848,57 +849,159 @@ __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_
           ca = fminf(fmaf(op, acc.w, ca), 1.f);
         }
       }
-      if (ca >= mp.early_term) break;
-      const int pos = __float_as_int(st[10 * kThreads]);
-      const int next = pos & 255, nseq = pos >> 8;
-      if (next >= nseq) break;
-      st[10 * kThreads] = __int_as_float(pos + 1);
-      const uint32_t word = (uint32_t)__float_as_int(st[(next < 8 ? 4 : 6) * kThreads]);
-      const int d = (int)((word >> (4 * (next & 7))) & 15u);
-      const DomainDev &dm = doms[d];
-      float t0, t1;
-      slab(dm, r, t0, t1);
-      const float covered = st[5 * kThreads];
-      bt0 = fmaxf(t0, covered);
-      bt1 = fminf(t1, st[7 * kThreads]);
-      st[5 * kThreads] = fmaxf(covered, bt1);
-      thr = mp.early_term < 1.f ? (mp.early_term - ca) / (1.f - ca) : 2.f;
-      acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      int pos = __float_as_int(st[10 * kThreads]);
+      if (!(ca >= mp.early_term) && (pos & 255) >= (pos >> 8 & 255) && (pos >> 24)) {
+        // order the next domains: those after the last one taken, sorted by
+        // insertion as they are found (indices ascend, so of equal entries the
+        // lower index stays first)
+        float last_t0 = -FLT_MAX;
+        int last_d = -1;
+        if ((pos >> 16 & 255) != 255) {
+          float t1;
+          last_d = pos >> 16 & 255;
+          slab(doms[last_d], r, last_t0, t1);
+        }
+        float at[kWalkDomains];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        A[a] = (r.o[a] - dm.origin[a]) * dm.inv_spacing[a];
-        B[a] = r.d[a] * dm.inv_spacing[a];
-        cmax[a] = dm.dims[a] - 2;
+        for (int i = 0; i < kWalkDomains; ++i) at[i] = INFINITY;
+        uint64_t ids = 0;
+        int found = 0;
+        for (uint64_t m = mask; m; m &= m - 1) {
+          const int d = __ffsll((long long)m) - 1;
+          float t0, t1;
+          if (!slab(doms[d], r, t0, t1)) continue;
+          if (!(t0 > last_t0 || (t0 == last_t0 && d > last_d))) continue;
+          ++found;
+          int place = 0;
+#pragma unroll
+          for (int i = kWalkDomains - 1; i >= 0; --i) {
+            place += at[i] <= t0 ? 1 : 0;
+            at[i] = fminf(at[i], i > 0 ? fmaxf(at[i > 0 ? i - 1 : 0], t0) : t0);
+          }
+          if (place < kWalkDomains) {
+            const uint64_t low = (1ull << (6 * place)) - 1ull;
+            ids = (ids & low) | (uint64_t)d << (6 * place) | (ids & ~low) << 6;
+          }
+        }
+        const int n = min(found, kWalkDomains);
+        constexpr int kHalf = 6 * kWalkDomains / 2;
+        st[4 * kThreads] = __int_as_float((int)(ids & ((1u << kHalf) - 1u)));
+        st[6 * kThreads] = __int_as_float((int)((ids >> kHalf) & ((1u << kHalf) - 1u)));
+        pos = n << 8 | (n ? (int)(ids >> (6 * n - 6)) & 63 : 255) << 16 | (found > kWalkDomains ? 1 << 24 : 0);
       }
-      sy = dm.nbrick[0] * BF;
-      sz = dm.nbrick[1] * sy;
-      bricks = dm.bricks;
-      k = 0;
-      last_off = -1;
-      started = true;
-      fresh = false;
+      const int next = pos & 255;
+      st[10 * kThreads] = __int_as_float(pos + 1);
+      if (ca >= mp.early_term || next >= (pos >> 8 & 255)) {
+        // no more: a place whose samples load nothing
+        live = false;
+        bt0 = bt1 = 0.f;
+        A[0] = A[1] = A[2] = B[0] = B[1] = B[2] = 0.f;
+        cmax[0] = cmax[1] = cmax[2] = 0;
+        last_off = 0;
+      } else {
+        const uint32_t word = (uint32_t)__float_as_int(st[(next < kWalkDomains / 2 ? 4 : 6) * kThreads]);
+        const int d = (int)((word >> (6 * (next < kWalkDomains / 2 ? next : next - kWalkDomains / 2))) & 63u);
+        const DomainDev &dm = doms[d];
+        float t0, t1;
+        slab(dm, r, t0, t1);
+        const float covered = st[5 * kThreads];
+        bt0 = fmaxf(t0, covered);
+        bt1 = fminf(t1, st[7 * kThreads]);
+        st[5 * kThreads] = fmaxf(covered, bt1);
+        thr = mp.early_term < 1.f ? (mp.early_term - ca) / (1.f - ca) : 2.f;
+        acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          A[a] = (r.o[a] - dm.origin[a]) * dm.inv_spacing[a];
+          B[a] = r.d[a] * dm.inv_spacing[a];
+          cmax[a] = dm.dims[a] - 2;
+        }
+        sy = dm.nbrick[0] * BF;
+        sz = dm.nbrick[1] * sy;
+        bricks = dm.bricks;
+        // steps of two cells and more: a brick holds so few samples that
+        // taking them costs less than passing over them
+        const float cells = dt * fmaxf(fabsf(B[0]), fmaxf(fabsf(B[1]), fabsf(B[2])));
+        hidden = any_hidden && cells < kSkipCells && *dm.any_empty ? d : -1;
+        k = 0;
+        last_off = -1;
+        brick = -1;
+        started = true;
+      }
     }
+    if (!__any_sync(warp, live)) break;
     float v[UNROLL];
     bool ok[UNROLL];
-    sample_cells<UNROLL, SH, false>(bricks, A, B, cmax, sy, sz, k, 0, dt, bt0, bt1, last_off, lc, v, ok);
+    sample_cells<UNROLL, 3, false>(bricks, A, B, cmax, sy, sz, k, 0, dt, bt0, bt1, last_off, lc, v, ok);
+    // the whole group if its last sample lies in the domain and no opacity on
+    // the way reaches the threshold; otherwise, once per ray and domain, again
+    // from the start, sample by sample
+    float4 all = acc;
+    float top = -INFINITY;
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u) {
-      if (!ok[u]) { count += k + u; fresh = true; break; }
       const float sc = __saturatef((v[u] - mp.scalar_min) * mp.inv_range);
-      float4 col;
-      if (mp.lut_filter == GVR_LUT_LINEAR) {
-        col = lut_fetch(lut, mp.lut_size, GVR_LUT_LINEAR, sc);
-      } else {
-        col = lut_nearest(lut, nm1, sc);
-      }
-      const float wa = (1.f - acc.w) * col.w;
-      acc.x = fmaf(wa, col.x, acc.x);
-      acc.y = fmaf(wa, col.y, acc.y);
-      acc.z = fmaf(wa, col.z, acc.z);
-      acc.w += wa;
-      if (acc.w >= thr) { count += k + u + 1; fresh = true; break; }
+      const float4 col = lut_color<LIN>(lut, mp, nm1, sc);
+      const float wa = (1.f - all.w) * col.w;
+      all.x = fmaf(wa, col.x, all.x);
+      all.y = fmaf(wa, col.y, all.y);
+      all.z = fmaf(wa, col.z, all.z);
+      all.w += wa;
+      top = u ? fmaxf(top, all.w) : all.w;
     }
-    k += UNROLL;
+    bool on = ok[UNROLL - 1] && !(top >= thr);
+    if (on) {
+      acc = all;
+      k += UNROLL;
+    } else if (live) {
+      fresh = true;
+      bool more = true;
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        if (more && ok[u]) {
+          const float sc = __saturatef((v[u] - mp.scalar_min) * mp.inv_range);
+          const float4 col = lut_color<LIN>(lut, mp, nm1, sc);
+          const float wa = (1.f - acc.w) * col.w;
+          acc.x = fmaf(wa, col.x, acc.x);
+          acc.y = fmaf(wa, col.y, acc.y);
+          acc.z = fmaf(wa, col.z, acc.z);
+          acc.w += wa;
+          ++k;
+          more = !(acc.w >= thr);
+        }
+      }
+      count += k;
+    }
+    // an offset is its brick's number times BF and a place below BF in it
+    if (on && hidden >= 0 && last_off / BF != brick) {
+      brick = last_off / BF;
+      const DomainDev &dm = doms[hidden];
+      int j = k - 1;      // a sample in `brick`
+      while (dm.brick_empty[brick]) {
+        // the samples up to one step before the ray leaves the brick lie in it
+        const float t = fmaf((float)j, dt, bt0);
+        float texit = bt1;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          if (B[a] != 0.f) {
+            const int b = max(0, min((int)fmaf(t, B[a], A[a]), cmax[a])) >> 3;
+            const float edge = B[a] > 0.f ? (float)min((b + 1) * 8, cmax[a] + 1) : (float)(b * 8);
+            texit = fminf(texit, __fdividef(edge - A[a], B[a]));
+          }
+        }
+        j = max((int)floorf(__fdividef(texit - bt0, dt)), j + 1);
+        const float tj = fmaf((float)j, dt, bt0);
+        if (!(tj < bt1)) break;
+        int b3[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) b3[a] = max(0, min((int)fmaf(tj, B[a], A[a]), cmax[a])) >> 3;
+        const int nb = (b3[2] * dm.nbrick[1] + b3[1]) * dm.nbrick[0] + b3[0];
+        if (nb == brick) break;
+        brick = nb;
+      }
+      k = max(j, k);
+    }
+    __syncwarp(warp);
   }
   const float crgb[3] = {st[0], st[kThreads], st[2 * kThreads]};
   const float cdepth = st[3 * kThreads];
@@ -915,20 +1018,23 @@ __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_
 template <int UNROLL, int MODE>
 __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, const ViewDev &view,
                                           const MarchParams &mp, const float4 *lut, int px, int py,
-                                          float4 &out, float &dep, float *g_state)
+                                          float4 &out, float &dep, float *g_state, bool any_hidden)
 {
-  if (MODE != kMarchHex && (mask & (mask - 1)) != 0 && mp.n_domains <= kUnifiedDomains) {
-    // two or more domains, every one a uniform vertex field in 8^3-cell
-    // bricks with no empty bricks to jump: the one-loop walk (a single
-    // domain has no crossing to wait at, and its own loop keeps fewer
-    // values live: 1.39 against 1.49 ms on the 513^3 field as one domain)
-    bool uni = true;
-    for (uint64_t m = mask; m; m &= m - 1) {
-      const DomainDev &dm = doms[__ffsll((long long)m) - 1];
-      uni = uni && dm.kind == GVR_DOMAIN_UNIFORM && dm.assoc == GVR_ASSOC_VERTEX && dm.bshift == 3 &&
-            !(mp.skip_empty && *dm.any_empty);
-    }
-    if (uni) return render_ray_unified<UNROLL, 3, MODE>(doms, mask, view, mp, lut, px, py, out, dep, g_state);
+  if (MODE != kMarchHex && mask) {
+    // domains that are all uniform vertex fields in 8^3-cell bricks, two or
+    // more of them or one with empty bricks to pass over: the one-loop walk (a
+    // single domain without has no crossing to wait at, and its own loop keeps
+    // fewer values live: 1.39 against 1.49 ms on the 513^3 field as one domain)
+    bool walk = doms[__ffsll((long long)mask) - 1].bshift == 3 && ((mask & (mask - 1)) != 0 || any_hidden);
+    if (MODE != kMarchUniform)
+      for (uint64_t m = mask; m; m &= m - 1) {
+        const DomainDev &dm = doms[__ffsll((long long)m) - 1];
+        walk = walk && dm.kind == GVR_DOMAIN_UNIFORM && dm.assoc == GVR_ASSOC_VERTEX && dm.bshift == 3;
+      }
+    if (walk)
+      return mp.lut_filter == GVR_LUT_LINEAR
+                 ? render_ray_unified<UNROLL, MODE, true>(doms, mask, view, mp, lut, px, py, out, dep, g_state, any_hidden)
+                 : render_ray_unified<UNROLL, MODE, false>(doms, mask, view, mp, lut, px, py, out, dep, g_state, any_hidden);
   }
   int count = 0;
   const Ray r = pixel_ray(view, mp, px, py);
@@ -988,14 +1094,21 @@ __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, 
         MODE == kMarchUniform || (dm.kind == GVR_DOMAIN_UNIFORM && dm.assoc == GVR_ASSOC_VERTEX);
     if (MODE == kMarchHex && dm.kind == GVR_DOMAIN_HEX)
       count += march_hex(dm, r, bt0, bt1, mp, lut, thr, acc);
-    else if (uniform_vertex && !(mp.skip_empty && *dm.any_empty))
-      count += dm.bshift == 3 ? march_uniform<UNROLL, 3>(dm, r, bt0, bt1, mp, lut, thr, acc)
-             : dm.bshift == 2 ? march_uniform<UNROLL, 2>(dm, r, bt0, bt1, mp, lut, thr, acc)
-                              : march_uniform<UNROLL, 4>(dm, r, bt0, bt1, mp, lut, thr, acc);
-    else if (uniform_vertex)
-      count += dm.bshift == 3 ? march_bricks<UNROLL, 3>(dm, r, bt0, bt1, mp, lut, thr, acc)
-             : dm.bshift == 2 ? march_bricks<UNROLL, 2>(dm, r, bt0, bt1, mp, lut, thr, acc)
-                              : march_bricks<UNROLL, 4>(dm, r, bt0, bt1, mp, lut, thr, acc);
+    else if (uniform_vertex && !(mp.skip_empty && *dm.any_empty)) {
+      if (mp.lut_filter == GVR_LUT_LINEAR)
+        count += dm.bshift == 3 ? march_uniform<UNROLL, 3, true>(dm, r, bt0, bt1, mp, lut, thr, acc)
+               : dm.bshift == 2 ? march_uniform<UNROLL, 2, true>(dm, r, bt0, bt1, mp, lut, thr, acc)
+                                : march_uniform<UNROLL, 4, true>(dm, r, bt0, bt1, mp, lut, thr, acc);
+      else
+        count += dm.bshift == 3 ? march_uniform<UNROLL, 3, false>(dm, r, bt0, bt1, mp, lut, thr, acc)
+               : dm.bshift == 2 ? march_uniform<UNROLL, 2, false>(dm, r, bt0, bt1, mp, lut, thr, acc)
+                                : march_uniform<UNROLL, 4, false>(dm, r, bt0, bt1, mp, lut, thr, acc);
+    } else if (uniform_vertex) {
+      // 8^3-cell bricks come here only next to other kinds of domains
+      count += MODE != kMarchUniform && dm.bshift == 3 ? march_bricks<UNROLL, 3>(dm, r, bt0, bt1, mp, lut, thr, acc)
+             : dm.bshift == 2                          ? march_bricks<UNROLL, 2>(dm, r, bt0, bt1, mp, lut, thr, acc)
+                                                       : march_bricks<UNROLL, 4>(dm, r, bt0, bt1, mp, lut, thr, acc);
+    }
     else {
       Partial part;
       if (MODE >= kMarchRect && dm.kind == GVR_DOMAIN_RECTILINEAR)
@@ -1054,7 +1167,9 @@ march_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
     uint32_t *dst = reinterpret_cast<uint32_t *>(doms);
     for (int i = threadIdx.x; i < words; i += kThreads) dst[i] = src[i];
   }
-  __syncthreads();
+  // whether any domain has empty bricks under this transfer function
+  const bool hidden = __syncthreads_or(mp.skip_empty && threadIdx.x < mp.n_domains &&
+                                       *g_domains[threadIdx.x].any_empty);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int px = tile_x * kTile + (warp % PX) * PW + (lane % PW);
@@ -1065,7 +1180,7 @@ march_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
     const uint64_t all = mp.n_domains >= 64 ? ~0ull : ((1ull << mp.n_domains) - 1ull);
     float4 out;
     float dep;
-    count = render_ray<UNROLL, MODE>(doms, all, view, mp, lut, px, py, out, dep, s_state);
+    count = render_ray<UNROLL, MODE>(doms, all, view, mp, lut, px, py, out, dep, s_state, hidden);
     const int64_t pix = (int64_t)py * mp.width + px;
     rgba[pix] = out;
     depth[pix] = dep;
@@ -1636,7 +1751,7 @@ layer_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
       const uint64_t all = mp.n_domains >= 64 ? ~0ull : ((1ull << mp.n_domains) - 1ull);
       float4 out;
       float dep;
-      count = render_ray<1, kMarchCells>(doms, all, view, mp, lut, px, py, out, dep, s_state);
+      count = render_ray<1, kMarchCells>(doms, all, view, mp, lut, px, py, out, dep, s_state, true);
       const int64_t pix = (int64_t)py * mp.width + px;
       rgba[pix] = out;
       depth[pix] = dep;
@@ -1911,6 +2026,8 @@ batch_kernel(const DomainDev *__restrict__ g_domains, const ViewDev *__restrict_
     uint32_t *dst = reinterpret_cast<uint32_t *>(doms);
     for (int i = threadIdx.x; i < words; i += kThreads) dst[i] = src[i];
   }
+  const bool hidden = __syncthreads_or(mp.skip_empty && threadIdx.x < mp.n_domains &&
+                                       *g_domains[threadIdx.x].any_empty);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_per_view = tiles_x * tiles_y;
   const long long total_tiles = (long long)tiles_per_view * n_views;
@@ -1947,7 +2064,7 @@ batch_kernel(const DomainDev *__restrict__ g_domains, const ViewDev *__restrict_
       if (px < mp.width && py < mp.height) {
         float4 out;
         float dep;
-        count += render_ray<UNROLL, MODE>(doms, mask, views[v], mp, lut, px, py, out, dep, s_state);
+        count += render_ray<UNROLL, MODE>(doms, mask, views[v], mp, lut, px, py, out, dep, s_state, hidden);
         const int64_t pix = (int64_t)v * pixels + (int64_t)py * mp.width + px;
         rgba[pix] = out;
         depth[pix] = dep;

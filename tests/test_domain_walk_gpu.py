@@ -101,3 +101,33 @@ def test_domain_walk_in_the_batch_kernel():
     for v in range(len(cams)):
         o, _, _ = osc.render(ocams[v], op)
         assert_parity(rgba[v], o)
+
+
+@pytest.mark.parametrize("parts", [(5, 4, 3), (11, 1, 1), (64, 1, 1), (1, 1, 1)])
+@pytest.mark.parametrize("where", ["outside", "inside"])
+@pytest.mark.parametrize("hidden,samples", [(False, 150), (True, 150), (True, 14), (True, 700)])
+def test_domain_walk_of_many_domains_and_empty_bricks(parts, where, hidden, samples):
+    """Up to the 64 domains a scene takes, more than ten of them on one ray
+    (the walk orders ten at a time), bricks that the transfer function hides,
+    steps above and below the two cells from which bricks are not passed over:
+    images and sample counts equal the staged march's exactly."""
+    wl = W.plain_small(n=65, width=88, height=72, samples=samples, parts=parts)
+    if hidden:
+        wl.alpha_pos, wl.alpha = np.array([0.0, 0.3, 1.0]), np.array([0.0, 0.0, 0.7])
+    cam = V.workload_camera(wl) if where == "outside" else inside_camera(wl)
+    if where == "inside":
+        cam.look_at[0], cam.look_at[1], cam.look_at[2] = wl.bounds[1], 0.5, cam.position[2]
+    p = V.workload_params(wl, lut=V.workload_renderer(wl).lut(True))
+    with S.Scene(0) as sc:
+        V.load_workload(sc, wl)
+        out = []
+        for staged in (0, 1):
+            sc.set_tuning(packet_w=8, unroll=2, min_blocks=4, staged=staged)
+            out.append(sc.render(cam, p, count_samples=True))
+        batch, _, n = sc.render_batch([cam], p, count_samples=True)
+    (g, gd, gn), (s, sd, sn) = out
+    np.testing.assert_array_equal(g, s)
+    np.testing.assert_array_equal(gd, sd)
+    np.testing.assert_array_equal(batch[0], g)
+    assert gn == sn == n
+    assert g[..., 3].max() > 0.02
