@@ -2090,8 +2090,9 @@ using MarchFn = void (*)(const DomainDev *, const ViewDev, const MarchParams, co
 template <int PW, int UNROLL, int MINB>
 MarchFn pick() { return march_kernel<PW, UNROLL, MINB>; }
 
-MarchFn select(const Tuning &t, int mode)
+MarchFn select(Tuning t, int mode)
 {
+  t.packet_w = packet_width(t, mode, false);
   // the hex path keeps a cell's eight coefficient records in registers: 2 or
   // 3 CTAs per SM (3 spills some 400 bytes and measured 1.5% faster)
   if (mode == kMarchHex) {
@@ -2109,15 +2110,10 @@ MarchFn select(const Tuning &t, int mode)
   if (mode == kMarchCells)
     return t.packet_w == 4 ? march_kernel<4, 2, 4, kMarchCells>
                            : (t.packet_w == 16 ? march_kernel<16, 2, 4, kMarchCells> : march_kernel<8, 2, 4, kMarchCells>);
-  // three samples per iteration exists only at 4 CTAs per SM (at 3 it
-  // measured slower than two)
-  if (t.unroll >= 4)
-    return t.min_blocks >= 4 ? (t.packet_w == 4 ? pick<4, 4, 4>() : pick<8, 4, 4>())
-                             : (t.packet_w == 4 ? pick<4, 4, 3>() : pick<8, 4, 3>());
-  if (t.unroll >= 3) {
-    if (t.min_blocks < 4) return t.packet_w == 4 ? pick<4, 3, 3>() : pick<8, 3, 3>();
-    return t.packet_w == 4 ? pick<4, 3, 4>() : (t.packet_w == 16 ? pick<16, 3, 4>() : pick<8, 3, 4>());
-  }
+  // three and four samples per iteration have kernels only at 3 CTAs per SM
+  // (one: four); with 64 registers they spill in the loop (1930 against 1437 us
+  // on the 513^3 field) and take two
+  if (t.unroll >= 3 && t.min_blocks < 4 && t.packet_w != 16) return t.packet_w == 4 ? pick<4, 4, 3>() : pick<8, 4, 3>();
   const int u = t.unroll >= 2 ? 2 : 1;
   const int m = t.min_blocks >= 4 ? 4 : 3;
   switch (t.packet_w) {
@@ -2307,8 +2303,9 @@ using BatchFn = void (*)(const DomainDev *, const ViewDev *, const int4 *, const
                          int, int, int, const float4 *, float4 *, float *, unsigned long long *,
                          unsigned int *);
 
-BatchFn select_batch(const Tuning &t, int mode)
+BatchFn select_batch(Tuning t, int mode)
 {
+  t.packet_w = packet_width(t, mode, true);
   if (mode == kMarchHex) return t.packet_w == 4 ? batch_kernel<4, 1, 2, kMarchHex> : batch_kernel<8, 1, 2, kMarchHex>;
   if (mode == kMarchRect)
     return t.packet_w == 4 ? batch_kernel<4, 2, 3, kMarchRect>
