@@ -383,6 +383,277 @@ __global__ void pixel_emit_kernel(const Partial *__restrict__ in, const uint32_t
   }
 }
 
+// ---------------------------------------------------------------------------
+// Slots: the dense path while the pixels are no more than twice the records.
+// Every pixel has kSlots places for record indices, which a record's atomic on
+// the pixel's count hands out directly, so there is no bucket offset to scan
+// for and no second pass over the records before they are blended; records
+// beyond the places hang on the pixel in a list. Bound by memory: the records
+// are read twice, once for their pixel ids (24-byte records, so every sector of
+// them) and once to blend, the index places stay in L2. 8 images of 1024^2 at
+// 80% cover (6.7M records, 161 MB): the histogram, three scans, bucket and emit
+// passes took 150 us of kernels, SLOT_FIG.
+// ---------------------------------------------------------------------------
+constexpr int kSlots = 8;
+constexpr int kSlotTile = 1024;   // pixels per CTA of the last two passes
+
+// Word-sized loads of a record, or 8-byte ones where the array is aligned.
+template <bool WIDE>
+__device__ __forceinline__ Partial load_partial(const Partial *__restrict__ p)
+{
+  Partial r;
+  if (WIDE) {
+    const uint2 *q = reinterpret_cast<const uint2 *>(p);
+    const uint2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+    r.pixel_id = (int32_t)a.x;
+    r.depth = __uint_as_float(a.y);
+    r.rgb[0] = __uint_as_float(b.x);
+    r.rgb[1] = __uint_as_float(b.y);
+    r.rgb[2] = __uint_as_float(c.x);
+    r.alpha = __uint_as_float(c.y);
+  } else {
+    r = *p;
+  }
+  return r;
+}
+
+// A record outside [lo, lo + r) (possible only when the caller gave the range)
+// is left out and sets *bad.
+__global__ void __launch_bounds__(256)
+slot_kernel(const Partial *__restrict__ in, int64_t n, int lo, int64_t r, uint32_t *__restrict__ cnt,
+            uint32_t *__restrict__ place, uint32_t *__restrict__ head, uint32_t *__restrict__ next,
+            unsigned *__restrict__ bad)
+{
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = (int64_t)__ldg(&in[i].pixel_id) - lo;
+    if (p < 0 || p >= r) {
+      atomicOr(bad, 1u);
+      continue;
+    }
+    const uint32_t s = atomicAdd(cnt + p, 1u);
+    if (s < kSlots) place[p * kSlots + s] = (uint32_t)i;
+    else next[i] = atomicExch(head + p, (uint32_t)i + 1u);   // 0 ends a list
+  }
+}
+
+// Pixels with one record and with more, per tile; the CTA that finishes last
+// turns the tiles' numbers into exclusive prefixes and writes the totals.
+__global__ void __launch_bounds__(256)
+slot_sums_kernel(const uint32_t *__restrict__ cnt, int64_t r, uint2 *__restrict__ sums, int tiles,
+                 unsigned *__restrict__ finished, uint32_t *__restrict__ totals)
+{
+  __shared__ uint2 part[8];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned one = 0, more = 0;
+  const int64_t p0 = (int64_t)blockIdx.x * kSlotTile;
+  for (int k = threadIdx.x; k < kSlotTile; k += 256) {
+    const uint32_t c = p0 + k < r ? cnt[p0 + k] : 0u;
+    one += c == 1;
+    more += c > 1;
+  }
+  one = __reduce_add_sync(0xffffffffu, one);
+  more = __reduce_add_sync(0xffffffffu, more);
+  if (lane == 0) part[warp] = make_uint2(one, more);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) {
+      one += part[w].x;
+      more += part[w].y;
+    }
+    sums[blockIdx.x] = make_uint2(one, more);
+    __threadfence();
+    last = atomicAdd(finished, 1u) == (unsigned)tiles - 1u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  uint2 run = make_uint2(0u, 0u);
+  for (int t0 = 0; t0 < tiles; t0 += 256) {
+    const int t = t0 + threadIdx.x;
+    const uint2 v = t < tiles ? __ldcg(sums + t) : make_uint2(0u, 0u);
+    uint2 x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned a = __shfl_up_sync(0xffffffffu, x.x, o), b = __shfl_up_sync(0xffffffffu, x.y, o);
+      if (lane >= o) {
+        x.x += a;
+        x.y += b;
+      }
+    }
+    if (lane == 31) part[warp] = x;
+    __syncthreads();
+    uint2 base = run;
+    for (int w = 0; w < 8; ++w) {
+      if (w < warp) {
+        base.x += part[w].x;
+        base.y += part[w].y;
+      }
+      run.x += part[w].x;
+      run.y += part[w].y;
+    }
+    if (t < tiles) sums[t] = make_uint2(base.x + x.x - v.x, base.y + x.y - v.y);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    totals[0] = run.x;
+    totals[1] = run.y;
+  }
+}
+
+// One thread per pixel: copy its record or blend its records in (depth, input
+// index) order. Up to kSlots records are loaded whole, so that each is read
+// once, and ordered by Batcher's odd-even merge network (19 exchanges) with
+// their colours; more are taken one by one, each the next in order among the
+// pixel's places and list. n_out (may be NULL) receives the count, -1 when a
+// record was outside the caller's range.
+template <bool WIDE>
+__global__ void __launch_bounds__(256)
+slot_emit_kernel(const Partial *__restrict__ in, const uint32_t *__restrict__ cnt,
+                 const uint32_t *__restrict__ place, const uint32_t *__restrict__ head,
+                 const uint32_t *__restrict__ next, const uint2 *__restrict__ sums, int64_t r,
+                 Partial *__restrict__ out, const uint32_t *__restrict__ totals, const unsigned *__restrict__ bad,
+                 int64_t *__restrict__ n_out, uint32_t *rows, int64_t n, uint32_t *__restrict__ used)
+{
+  __shared__ uint2 part[8];
+  __shared__ int n_deep;                    // pixels deeper than kLocalSort: place in the tile, output
+  __shared__ int deep[kSlotTile];
+  __shared__ uint32_t deep_out[kSlotTile];
+  __shared__ uint32_t row;
+  if (threadIdx.x == 0) n_deep = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t n_unique = totals[0];
+  if (n_out && blockIdx.x == 0 && threadIdx.x == 0)
+    *n_out = *bad ? -1 : (int64_t)n_unique + totals[1];
+  uint2 base = sums[blockIdx.x];
+  for (int k0 = 0; k0 < kSlotTile; k0 += 256) {
+    const int64_t p = (int64_t)blockIdx.x * kSlotTile + k0 + threadIdx.x;
+    const uint32_t c = p < r ? cnt[p] : 0u;
+    const unsigned ones = __ballot_sync(0xffffffffu, c == 1), mores = __ballot_sync(0xffffffffu, c > 1);
+    if (lane == 0) part[warp] = make_uint2(__popc(ones), __popc(mores));
+    __syncthreads();
+    uint32_t upos = base.x + __popc(ones & ((1u << lane) - 1u)), mpos = base.y + __popc(mores & ((1u << lane) - 1u));
+    for (int w = 0; w < 8; ++w) {
+      const uint2 q = part[w];
+      if (w < warp) {
+        upos += q.x;
+        mpos += q.y;
+      }
+      base.x += q.x;
+      base.y += q.y;
+    }
+    __syncthreads();
+    if (c == 0) continue;
+    const uint32_t *seg = place + p * kSlots;
+    if (c == 1) {
+      out[upos] = load_partial<WIDE>(in + seg[0]);
+      continue;
+    }
+    Partial res;
+    if (c <= kSlots) {
+      const uint4 s0 = *reinterpret_cast<const uint4 *>(seg), s1 = *reinterpret_cast<const uint4 *>(seg + 4);
+      uint32_t idx[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+      uint32_t key[8];
+      Partial rec[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if ((uint32_t)j < c) rec[j] = load_partial<WIDE>(in + idx[j]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if ((uint32_t)j < c) {
+          key[j] = order_bits(rec[j].depth);
+        } else {
+          // sorts last, and blends as nothing
+          key[j] = 0xffffffffu;
+          idx[j] = 0xffffffffu;
+          rec[j] = Partial{0, 0.f, {0.f, 0.f, 0.f}, 0.f};
+        }
+      }
+      auto cx = [&](int a, int b) {
+        const bool swap = before(key[b], idx[b], key[a], idx[a]);
+        const uint32_t ka = key[a], ia = idx[a];
+        const Partial ra = rec[a];
+        key[a] = swap ? key[b] : ka;
+        idx[a] = swap ? idx[b] : ia;
+        key[b] = swap ? ka : key[b];
+        idx[b] = swap ? ia : idx[b];
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          rec[a].rgb[m] = swap ? rec[b].rgb[m] : ra.rgb[m];
+          rec[b].rgb[m] = swap ? ra.rgb[m] : rec[b].rgb[m];
+        }
+        rec[a].alpha = swap ? rec[b].alpha : ra.alpha;
+        rec[b].alpha = swap ? ra.alpha : rec[b].alpha;
+      };
+      cx(0, 1); cx(2, 3); cx(4, 5); cx(6, 7);
+      cx(0, 2); cx(1, 3); cx(4, 6); cx(5, 7);
+      cx(1, 2); cx(5, 6);
+      cx(0, 4); cx(1, 5); cx(2, 6); cx(3, 7);
+      cx(2, 4); cx(3, 5);
+      cx(1, 2); cx(3, 4); cx(5, 6);
+      res = rec[0];
+      res.pixel_id = __ldg(&in[idx[0]].pixel_id);
+      res.depth = __ldg(&in[idx[0]].depth);
+#pragma unroll
+      for (int j = 1; j < 8; ++j)
+        if ((uint32_t)j < c) blend_into(res, rec[j]);
+    } else if (c <= kLocalSort) {
+      uint32_t key[kLocalSort], idx[kLocalSort];
+      uint32_t held = 0;
+      auto insert = [&](uint32_t i) {
+        const uint32_t k = order_bits(__ldg(&in[i].depth));
+        uint32_t q = held++;
+        while (q > 0 && before(k, i, key[q - 1], idx[q - 1])) {
+          key[q] = key[q - 1];
+          idx[q] = idx[q - 1];
+          --q;
+        }
+        key[q] = k;
+        idx[q] = i;
+      };
+      for (int m = 0; m < kSlots; ++m) insert(seg[m]);
+      for (uint32_t t = head[p]; t; t = next[t - 1]) insert(t - 1);
+      res = load_partial<WIDE>(in + idx[0]);
+      for (uint32_t j = 1; j < c; ++j) blend_into(res, load_partial<WIDE>(in + idx[j]));
+    } else {
+      const int d = atomicAdd(&n_deep, 1);
+      deep[d] = k0 + (int)threadIdx.x;
+      deep_out[d] = n_unique + mpos;
+      continue;
+    }
+    out[n_unique + mpos] = res;
+  }
+  __syncthreads();
+  for (int d = 0; d < n_deep; ++d) {
+    const int64_t p = (int64_t)blockIdx.x * kSlotTile + deep[d];
+    const uint32_t c = cnt[p];
+    if (threadIdx.x == 0) {
+      row = atomicAdd(used, c);
+      uint32_t m = row;
+      for (int j = 0; j < kSlots; ++j) rows[m++] = place[p * kSlots + j];
+      for (uint32_t t = head[p]; t; t = next[t - 1]) rows[m++] = t - 1;
+    }
+    __syncthreads();
+    const uint32_t *from = rows + row;
+    uint32_t *sorted = rows + n + row;
+    for (uint32_t j = threadIdx.x; j < c; j += 256) {
+      const uint32_t i = from[j], k = order_bits(__ldg(&in[i].depth));
+      uint32_t rank = 0;
+      for (uint32_t q = 0; q < c; ++q) rank += before(order_bits(__ldg(&in[from[q]].depth)), from[q], k, i);
+      sorted[rank] = i;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      Partial res = load_partial<WIDE>(in + sorted[0]);
+      for (uint32_t j = 1; j < c; ++j) blend_into(res, load_partial<WIDE>(in + sorted[j]));
+      out[deep_out[d]] = res;
+    }
+    __syncthreads();
+  }
+}
+
 int grid_of(int64_t n)
 {
   const int64_t b = (n + 255) / 256;
@@ -412,6 +683,43 @@ size_t sorted_bytes(int64_t n)
 {
   return 256 * 12 + (2 * sizeof(uint64_t) + 6 * sizeof(uint32_t)) * (size_t)n +
          (sort_scratch_words(n) + scan_scratch_words(n) + 2) * sizeof(uint32_t);
+}
+
+// Whether the slots serve: their places are read for every pixel, and take 32
+// bytes of scratch each.
+bool use_slots(int64_t n, int64_t r) { return r <= 2 * n && (r + kSlotTile - 1) / kSlotTile < ((int64_t)1 << 30); }
+
+size_t slot_bytes(int64_t n, int64_t r)
+{
+  return 256 * 9 + ((2 + kSlots) * (size_t)r + 3 * (size_t)n + 2 * (size_t)((r + kSlotTile - 1) / kSlotTile) + 8) *
+                       sizeof(uint32_t);
+}
+
+// Dense pixel ids, no more than twice as many as records: slots, tile sums,
+// per-pixel emit. n_out: see slot_emit_kernel.
+cudaError_t composite_slots(const Partial *in, int64_t n, int lo, int64_t r, Partial *out, Arena &a,
+                            uint32_t *totals, int64_t *n_out, cudaStream_t st)
+{
+  const int tiles = (int)((r + kSlotTile - 1) / kSlotTile);
+  uint32_t *place = a.take<uint32_t>(kSlots * (size_t)r);
+  uint32_t *next = a.take<uint32_t>(n);
+  uint32_t *rows = a.take<uint32_t>(2 * (size_t)n);   // deep pixels' records, then in order
+  uint2 *sums = a.take<uint2>(tiles);
+  // counts, list heads and the three words are cleared together
+  uint32_t *cnt = a.take<uint32_t>(2 * (size_t)r + 3), *head = cnt + r;
+  unsigned *bad = head + r, *finished = bad + 1, *used = bad + 2;
+  cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (2 * (size_t)r + 3), st);
+  if (e != cudaSuccess) return e;
+  slot_kernel<<<grid_of(n), 256, 0, st>>>(in, n, lo, r, cnt, place, head, next, bad);
+  slot_sums_kernel<<<(unsigned)tiles, 256, 0, st>>>(cnt, r, sums, tiles, finished, totals);
+  if (((uintptr_t)in & 7) == 0)
+    slot_emit_kernel<true><<<(unsigned)tiles, 256, 0, st>>>(in, cnt, place, head, next, sums, r, out, totals, bad, n_out,
+                                                               rows, n, used);
+  else
+    slot_emit_kernel<false><<<(unsigned)tiles, 256, 0, st>>>(in, cnt, place, head, next, sums, r, out, totals, bad, n_out,
+                                                               rows, n, used);
+  count_launch(3);
+  return cudaGetLastError();
 }
 
 // Dense pixel ids: histogram, bucket, per-pixel emit.
@@ -529,13 +837,15 @@ extern "C" int gvr_composite_partials(const gvr_partial *partials, int64_t n, gv
     const int lo = (int)(hm[0] ^ 0x80000000u), hi = (int)(hm[1] ^ 0x80000000u);
     const int64_t r = (int64_t)hi - lo + 1;
     const bool dense = r <= 2 * n + 65536 && r < ((int64_t)1 << 31);
-    const size_t bytes = dense ? dense_bytes(n, r) : sorted_bytes(n);
+    const bool slots = dense && use_slots(n, r);
+    const size_t bytes = slots ? slot_bytes(n, r) : dense ? dense_bytes(n, r) : sorted_bytes(n);
     CP_TRY(scratch_alloc((void **)&arena.base, bytes, st), "allocate scratch");
     totals = arena.take<uint32_t>(2);
     // the range was measured, so no record is outside it: mm[0] serves as
     // the (unused) flag word
-    CP_TRY(dense ? composite_dense(d_in, n, lo, r, d_out, arena, totals, mm, st)
-                 : composite_sorted(d_in, n, d_out, arena, totals, st),
+    CP_TRY(slots   ? composite_slots(d_in, n, lo, r, d_out, arena, totals, nullptr, st)
+           : dense ? composite_dense(d_in, n, lo, r, d_out, arena, totals, mm, st)
+                   : composite_sorted(d_in, n, d_out, arena, totals, st),
            "composite");
     CP_TRY(cudaMemcpyAsync(ht, totals, sizeof(ht), cudaMemcpyDeviceToHost, st), "read counts");
     CP_TRY(cudaStreamSynchronize(st), "composite");
@@ -574,9 +884,16 @@ extern "C" int gvr_composite_partials_async(const gvr_partial *partials, int64_t
     return e == cudaSuccess ? GVR_OK : cuda_error(e, "composite");
   }
   Arena arena;
-  e = scratch_alloc((void **)&arena.base, dense_bytes(n, r), st);
+  const bool slots = use_slots(n, r);
+  e = scratch_alloc((void **)&arena.base, slots ? slot_bytes(n, r) : dense_bytes(n, r), st);
   if (e != cudaSuccess) return cuda_error(e, "allocate scratch");
   uint32_t *totals = arena.take<uint32_t>(2);
+  if (slots) {
+    e = composite_slots(reinterpret_cast<const Partial *>(partials), n, pixel_lo, r, reinterpret_cast<Partial *>(out),
+                        arena, totals, n_out, st);
+    cudaFreeAsync(arena.base, st);
+    return e == cudaSuccess ? GVR_OK : cuda_error(e, "composite");
+  }
   unsigned *bad = arena.take<unsigned>(1);
   e = cudaMemsetAsync(bad, 0, sizeof(unsigned), st);
   if (e == cudaSuccess)
