@@ -86,8 +86,8 @@ struct DomainDev {
 // iteration and the CTAs per SM the register budget targets (3, 4).
 struct Tuning {
   int packet_w = 0;         // 0 = until one is set, packet_width()'s
-  int unroll = 2;
-  int min_blocks = 4;
+  int unroll = 0;           // 0 = until set, by the frame's size (see select in gvr_march.cu)
+  int min_blocks = 0;
   int tiles_per_item = 1;   // batch path: 16x16 tiles per work-queue item
   int staged = 0;           // plain path: stage bricks in shared memory (uniform vertex scenes)
   int tile_order = 0;       // plain path: 0 = tiles nearest the image centre first,
