@@ -385,14 +385,17 @@ __global__ void pixel_emit_kernel(const Partial *__restrict__ in, const uint32_t
 
 // ---------------------------------------------------------------------------
 // Slots: the dense path while the pixels are no more than twice the records.
-// Every pixel has kSlots places for record indices, which a record's atomic on
-// the pixel's count hands out directly, so there is no bucket offset to scan
+// Every pixel has kSlots places for record indices (place s of all pixels
+// together: neighbouring records mostly take the same place of neighbouring
+// pixels), which a record's atomic on the pixel's count hands out directly, so there is no bucket offset to scan
 // for and no second pass over the records before they are blended; records
 // beyond the places hang on the pixel in a list. Bound by memory: the records
 // are read twice, once for their pixel ids (24-byte records, so every sector of
 // them) and once to blend, the index places stay in L2. 8 images of 1024^2 at
 // 80% cover (6.7M records, 161 MB): the histogram, three scans, bucket and emit
-// passes took 150 us of kernels, SLOT_FIG.
+// passes took 150 us of kernels, these three 99: 38 (4.6 TB/s), 7 and 51, the
+// last waiting for its records (55 with a barrier between a thread's pixels, 61
+// at 3 CTAs per SM, 92 at 5, where it spills).
 // ---------------------------------------------------------------------------
 constexpr int kSlots = 8;
 constexpr int kSlotTile = 1024;   // pixels per CTA of the last two passes
@@ -432,7 +435,7 @@ slot_kernel(const Partial *__restrict__ in, int64_t n, int lo, int64_t r, uint32
       continue;
     }
     const uint32_t s = atomicAdd(cnt + p, 1u);
-    if (s < kSlots) place[p * kSlots + s] = (uint32_t)i;
+    if (s < kSlots) place[s * r + p] = (uint32_t)i;
     else next[i] = atomicExch(head + p, (uint32_t)i + 1u);   // 0 ends a list
   }
 }
@@ -509,14 +512,15 @@ slot_sums_kernel(const uint32_t *__restrict__ cnt, int64_t r, uint2 *__restrict_
 // pixel's places and list. n_out (may be NULL) receives the count, -1 when a
 // record was outside the caller's range.
 template <bool WIDE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 slot_emit_kernel(const Partial *__restrict__ in, const uint32_t *__restrict__ cnt,
                  const uint32_t *__restrict__ place, const uint32_t *__restrict__ head,
                  const uint32_t *__restrict__ next, const uint2 *__restrict__ sums, int64_t r,
                  Partial *__restrict__ out, const uint32_t *__restrict__ totals, const unsigned *__restrict__ bad,
                  int64_t *__restrict__ n_out, uint32_t *rows, int64_t n, uint32_t *__restrict__ used)
 {
-  __shared__ uint2 part[8];
+  constexpr int kRows = kSlotTile / 256;    // pixels per thread
+  __shared__ uint2 part[kRows][8];
   __shared__ int n_deep;                    // pixels deeper than kLocalSort: place in the tile, output
   __shared__ int deep[kSlotTile];
   __shared__ uint32_t deep_out[kSlotTile];
@@ -527,35 +531,45 @@ slot_emit_kernel(const Partial *__restrict__ in, const uint32_t *__restrict__ cn
   const uint32_t n_unique = totals[0];
   if (n_out && blockIdx.x == 0 && threadIdx.x == 0)
     *n_out = *bad ? -1 : (int64_t)n_unique + totals[1];
-  uint2 base = sums[blockIdx.x];
-  for (int k0 = 0; k0 < kSlotTile; k0 += 256) {
-    const int64_t p = (int64_t)blockIdx.x * kSlotTile + k0 + threadIdx.x;
-    const uint32_t c = p < r ? cnt[p] : 0u;
+  // the counts and output slots of all of a thread's pixels first, so that
+  // nothing is waited for between them
+  __shared__ uint32_t counts[kRows][256];
+#pragma unroll
+  for (int q = 0; q < kRows; ++q) {
+    const int64_t p = (int64_t)blockIdx.x * kSlotTile + q * 256 + threadIdx.x;
+    const uint32_t c = p < r ? __ldg(cnt + p) : 0u;
     const unsigned ones = __ballot_sync(0xffffffffu, c == 1), mores = __ballot_sync(0xffffffffu, c > 1);
-    if (lane == 0) part[warp] = make_uint2(__popc(ones), __popc(mores));
-    __syncthreads();
-    uint32_t upos = base.x + __popc(ones & ((1u << lane) - 1u)), mpos = base.y + __popc(mores & ((1u << lane) - 1u));
+    counts[q][threadIdx.x] = c;
+    if (lane == 0) part[q][warp] = make_uint2(__popc(ones), __popc(mores));
+  }
+  __syncthreads();
+  uint2 base = sums[blockIdx.x];
+#pragma unroll 1
+  for (int q = 0; q < kRows; ++q) {
+    const int64_t p = (int64_t)blockIdx.x * kSlotTile + q * 256 + threadIdx.x;
+    const uint32_t c = counts[q][threadIdx.x];
+    uint32_t upos = base.x + __popc(__ballot_sync(0xffffffffu, c == 1) & ((1u << lane) - 1u));
+    uint32_t mpos = base.y + __popc(__ballot_sync(0xffffffffu, c > 1) & ((1u << lane) - 1u));
     for (int w = 0; w < 8; ++w) {
-      const uint2 q = part[w];
+      const uint2 v = part[q][w];
       if (w < warp) {
-        upos += q.x;
-        mpos += q.y;
+        upos += v.x;
+        mpos += v.y;
       }
-      base.x += q.x;
-      base.y += q.y;
+      base.x += v.x;
+      base.y += v.y;
     }
-    __syncthreads();
     if (c == 0) continue;
-    const uint32_t *seg = place + p * kSlots;
+    const uint32_t *seg = place + p;
     if (c == 1) {
       out[upos] = load_partial<WIDE>(in + seg[0]);
       continue;
     }
     Partial res;
     if (c <= kSlots) {
-      const uint4 s0 = *reinterpret_cast<const uint4 *>(seg), s1 = *reinterpret_cast<const uint4 *>(seg + 4);
-      uint32_t idx[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-      uint32_t key[8];
+      uint32_t idx[8], key[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) idx[j] = (uint32_t)j < c ? __ldg(seg + j * r) : 0u;
       Partial rec[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j)
@@ -613,13 +627,13 @@ slot_emit_kernel(const Partial *__restrict__ in, const uint32_t *__restrict__ cn
         key[q] = k;
         idx[q] = i;
       };
-      for (int m = 0; m < kSlots; ++m) insert(seg[m]);
+      for (int m = 0; m < kSlots; ++m) insert(seg[m * r]);
       for (uint32_t t = head[p]; t; t = next[t - 1]) insert(t - 1);
       res = load_partial<WIDE>(in + idx[0]);
       for (uint32_t j = 1; j < c; ++j) blend_into(res, load_partial<WIDE>(in + idx[j]));
     } else {
       const int d = atomicAdd(&n_deep, 1);
-      deep[d] = k0 + (int)threadIdx.x;
+      deep[d] = q * 256 + (int)threadIdx.x;
       deep_out[d] = n_unique + mpos;
       continue;
     }
@@ -632,7 +646,7 @@ slot_emit_kernel(const Partial *__restrict__ in, const uint32_t *__restrict__ cn
     if (threadIdx.x == 0) {
       row = atomicAdd(used, c);
       uint32_t m = row;
-      for (int j = 0; j < kSlots; ++j) rows[m++] = place[p * kSlots + j];
+      for (int j = 0; j < kSlots; ++j) rows[m++] = place[j * r + p];
       for (uint32_t t = head[p]; t; t = next[t - 1]) rows[m++] = t - 1;
     }
     __syncthreads();
