@@ -63,6 +63,7 @@ struct DiffParams {
   int n_seg;       // checkpoint segments per ray
   int lut_copies;  // backward: LUT-gradient copies in global memory (CTA c uses c % copies)
   int64_t n_rays;  // views x height x width
+  int packets;     // rays numbered by 8 x 4-pixel packets (see ray_number)
   int64_t v_offset;  // start of the per-sample scalar cache in the workspace
   float sample_dist;
   float scalar_min;
@@ -103,34 +104,49 @@ __device__ __forceinline__ bool diff_ray(const ViewDev &view, const DiffGrid &g,
   return t1 > t0;
 }
 
-// Cell (linear index of its corner 000) and trilinear weights of sample t.
-__device__ __forceinline__ int64_t diff_cell(const DiffGrid &g, const float A[3], const float B[3],
-                                             float t, float w[3])
+// Number of a ray in the workspace: where the image is whole 8 x 4-pixel
+// packets, a warp's 32 rays one after the other, so that the scalars it stores
+// and loads for a sample are one 128-byte line and not four pieces of rows;
+// otherwise the pixels row by row.
+__device__ __forceinline__ int64_t ray_number(const DiffParams &p, int v, int px, int py)
+{
+  if (!p.packets) return ((int64_t)v * p.height + py) * p.width + px;
+  const int packet = (py >> 2) * (p.width >> 3) + (px >> 3);
+  return (int64_t)v * p.width * p.height + 32 * (int64_t)packet + ((py & 3) * 8 + (px & 7));
+}
+
+// Cell (linear index of its corner 000, of type I: int where the field has
+// fewer than 2^31 nodes) and trilinear weights of sample t.
+template <typename I>
+__device__ __forceinline__ I diff_cell(const DiffGrid &g, const float A[3], const float B[3],
+                                       float t, float w[3])
 {
   int c[3];
   for (int a = 0; a < 3; ++a) {
     const float gg = fmaf(t, B[a], A[a]);
-    c[a] = max(0, min((int)gg, g.dims[a] - 2));
+    c[a] = __vimin_s32_relu((int)gg, g.dims[a] - 2);   // max(0, min)
     w[a] = gg - (float)c[a];
   }
-  return ((int64_t)c[2] * g.dims[1] + c[1]) * g.dims[0] + c[0];
+  return ((I)c[2] * g.dims[1] + c[1]) * g.dims[0] + c[0];
 }
 
 // The 8 corners of the cell at base: (x, y, z) bits of the index are
 // (1, 2, 4).
+template <typename I>
 __device__ __forceinline__ void diff_corners(const float *__restrict__ f, const DiffGrid &g,
-                                             int64_t base, float c[8])
+                                             I base, float c[8])
 {
-  const int64_t sy = g.dims[0], sz = (int64_t)g.dims[0] * g.dims[1];
+  const I sy = g.dims[0], sz = (I)g.dims[0] * g.dims[1];
   const float *p = f + base;
   c[0] = __ldg(p);
   c[1] = __ldg(p + 1);
   c[2] = __ldg(p + sy);
   c[3] = __ldg(p + sy + 1);
-  c[4] = __ldg(p + sz);
-  c[5] = __ldg(p + sz + 1);
-  c[6] = __ldg(p + sz + sy);
-  c[7] = __ldg(p + sz + sy + 1);
+  p += sz;
+  c[4] = __ldg(p);
+  c[5] = __ldg(p + 1);
+  c[6] = __ldg(p + sy);
+  c[7] = __ldg(p + sy + 1);
 }
 
 __device__ __forceinline__ float diff_interp(const float c[8], const float w[3])
@@ -151,9 +167,10 @@ __device__ __forceinline__ float lut_alpha(const float *lut_a, const DiffParams 
   return lerp2(lut_a[i0], lut_a[i0 + 1], x - (float)i0);
 }
 
-// Linear LUT lookup at scalar v; also returns the entry index i0 and weight.
+// Linear LUT lookup at scalar v; also returns the entry index i0, the weight
+// and the difference of entries i0 + 1 and i0.
 __device__ __forceinline__ float4 diff_lut(const float4 *lut, const DiffParams &p, float v,
-                                           float &s_raw, int &i0, float &wl)
+                                           float &s_raw, int &i0, float &wl, float4 &step)
 {
   s_raw = (v - p.scalar_min) * p.inv_range;
   const float s = __saturatef(s_raw);
@@ -161,10 +178,11 @@ __device__ __forceinline__ float4 diff_lut(const float4 *lut, const DiffParams &
   i0 = min((int)x, p.lut_size - 2);
   wl = x - (float)i0;
   const float4 a = lut[i0], b = lut[i0 + 1];
-  return make_float4(lerp2(a.x, b.x, wl), lerp2(a.y, b.y, wl), lerp2(a.z, b.z, wl),
-                     lerp2(a.w, b.w, wl));
+  step = make_float4(b.x - a.x, b.y - a.y, b.z - a.z, b.w - a.w);
+  return make_float4(fmaf(wl, step.x, a.x), fmaf(wl, step.y, a.y), fmaf(wl, step.z, a.z), fmaf(wl, step.w, a.w));
 }
 
+template <typename I>
 __global__ void __launch_bounds__(256)
 diff_forward(const float *__restrict__ field, const DiffGrid g, const DiffViews views,
              const DiffParams p, const float4 *__restrict__ g_lut, float4 *__restrict__ rgba,
@@ -178,7 +196,6 @@ diff_forward(const float *__restrict__ field, const DiffGrid g, const DiffViews 
   const int py = blockIdx.y * 16 + (warp >> 1) * 4 + (lane >> 3);
   const int v = blockIdx.z;
   if (px >= p.width || py >= p.height) return;
-  const int64_t ray = ((int64_t)v * p.height + py) * p.width + px;
   float o[3], d[3], t0, t1;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   if (diff_ray(views.v[v], g, p, px, py, o, d, t0, t1)) {
@@ -187,27 +204,31 @@ diff_forward(const float *__restrict__ field, const DiffGrid g, const DiffViews 
       A[a] = (o[a] - g.origin[a]) * g.inv_spacing[a];
       B[a] = d[a] * g.inv_spacing[a];
     }
+    const int64_t ray = ray_number(p, v, px, py);
+    float *check = ws ? ws + ray * p.n_seg : nullptr;     // transmittance at the next segment's start
+    float *scalar = ws ? ws + p.v_offset + ray : nullptr; // the next sample's scalar
     // corners of the last cell loaded, reused while samples stay in it
-    int64_t last = -1;
+    I last = -1;
     float cc[8];
     for (int k = 0;; ++k) {
       const float t = fmaf((float)k, p.sample_dist, t0);
       if (!(t < t1)) break;
-      if (ws) {
-        // transmittance checkpoint at each segment start, scalar of every sample
-        if ((k % kDiffK) == 0) ws[ray * p.n_seg + k / kDiffK] = 1.f - acc.w;
-      }
+      if (ws && (k % kDiffK) == 0) *check++ = 1.f - acc.w;
       float w[3];
-      const int64_t base = diff_cell(g, A, B, t, w);
+      const I base = diff_cell<I>(g, A, B, t, w);
       if (base != last) {
-        diff_corners(field, g, base, cc);
+        diff_corners<I>(field, g, base, cc);
         last = base;
       }
       const float val = diff_interp(cc, w);
-      if (ws) ws[p.v_offset + (int64_t)k * p.n_rays + ray] = val;
+      if (ws) {
+        *scalar = val;
+        scalar += p.n_rays;
+      }
       float s_raw, wl;
       int i0;
-      const float4 c = diff_lut(lut, p, val, s_raw, i0, wl);
+      float4 step;
+      const float4 c = diff_lut(lut, p, val, s_raw, i0, wl, step);
       const float wa = (1.f - acc.w) * c.w;
       acc.x = fmaf(wa, c.x, acc.x);
       acc.y = fmaf(wa, c.y, acc.y);
@@ -215,35 +236,43 @@ diff_forward(const float *__restrict__ field, const DiffGrid g, const DiffViews 
       acc.w += wa;
     }
   }
-  rgba[ray] = acc;
+  rgba[((int64_t)v * p.height + py) * p.width + px] = acc;
 }
 
 // Add g8 (the gradients of one cell's eight corners) to the field gradient.
 // Warp-aggregated in pairs: lanes 2i and 2i + 1 (neighbouring pixels in x)
-// that flush the same cell at the same step add their sums first, so one
-// atomic covers both. Measured against pooling whole peer sets
-// (__match_any_sync, then shuffles) and against 2x2 / 4x2 pixel groups,
-// pairs were fastest: wider groups cost more shuffles than they save
-// atomics. The sums go to the corner-quad buffer gq (one float4 per cell
-// base: corners (x, y), (x+1, y), (x, y+1), (x+1, y+1) of one z layer), so a
-// flush is two 16-byte vector atomics, each in one sector; fold_quads adds
-// the quads into the node gradient afterwards. Called by all lanes.
+// that flush the same cell at the same step add their sums first, the even
+// lane the corners of the lower z layer and the odd lane those of the upper, so
+// that four values change hands and each lane makes one atomic. Measured
+// against pooling whole peer sets (__match_any_sync, then shuffles) and against
+// 2x2 / 4x2 pixel groups, pairs were fastest: wider groups cost more shuffles
+// than they save atomics. The sums go to the corner-quad buffer gq (one float4
+// per cell base: corners (x, y), (x+1, y), (x, y+1), (x+1, y+1) of one z
+// layer), so a flush is 16-byte vector atomics, each in one sector; fold_quads
+// adds the quads into the node gradient afterwards. Called by all lanes.
+template <typename I>
 __device__ __forceinline__ void flush_cell(float4 *__restrict__ gq, const DiffGrid &g,
-                                           int64_t base, const float g8[8], bool active)
+                                           I base, const float g8[8], bool active)
 {
   const int lane = threadIdx.x & 31;
-  const int64_t ob = __shfl_xor_sync(0xffffffffu, active ? base : -1 - (int64_t)lane, 1);
-  const bool pair = active && ob == base;
-  float s[8];
+  const I mine = active ? base : (I)(-1 - lane);
+  const bool pair = __shfl_xor_sync(0xffffffffu, mine, 1) == mine;
+  const bool odd = lane & 1;
+  float s[4];
 #pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const float x = __shfl_xor_sync(0xffffffffu, g8[m], 1);
-    s[m] = g8[m] + (pair ? x : 0.f);
+  for (int m = 0; m < 4; ++m) {
+    // what this lane keeps, and what it hands over
+    const float keep = odd ? g8[4 + m] : g8[m];
+    s[m] = keep + __shfl_xor_sync(0xffffffffu, odd ? g8[m] : g8[4 + m], 1);
   }
-  if (!active || (pair && (lane & 1))) return;
-  const int64_t sz = (int64_t)g.dims[0] * g.dims[1];
-  atomicAdd(gq + base, make_float4(s[0], s[1], s[2], s[3]));
-  atomicAdd(gq + base + sz, make_float4(s[4], s[5], s[6], s[7]));
+  if (!active) return;
+  float4 *lower = gq + base, *upper = lower + (I)g.dims[0] * g.dims[1];
+  if (pair) {
+    atomicAdd(odd ? upper : lower, make_float4(s[0], s[1], s[2], s[3]));
+  } else {
+    atomicAdd(lower, make_float4(g8[0], g8[1], g8[2], g8[3]));
+    atomicAdd(upper, make_float4(g8[4], g8[5], g8[6], g8[7]));
+  }
 }
 
 // grad[i] += quads whose corners include node i: its own quad's (x, y)
@@ -275,6 +304,7 @@ __device__ __forceinline__ void flush_lut4(float *copy, int li, float (&lg)[8])
   for (int m = 0; m < 8; ++m) lg[m] = 0.f;
 }
 
+template <typename I>
 __global__ void __launch_bounds__(256)
 diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews views,
               const DiffParams p, const float4 *__restrict__ g_lut,
@@ -309,8 +339,8 @@ diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews
   float A[3] = {0.f, 0.f, 0.f}, B[3] = {0.f, 0.f, 0.f};
   int64_t ray = 0;
   if (hit) {
-    ray = ((int64_t)v * p.height + py) * p.width + px;
-    gr = grad_rgba[ray];
+    ray = ray_number(p, v, px, py);
+    gr = grad_rgba[((int64_t)v * p.height + py) * p.width + px];
     for (int a = 0; a < 3; ++a) {
       A[a] = (o[a] - g.origin[a]) * g.inv_spacing[a];
       B[a] = d[a] * g.inv_spacing[a];
@@ -323,11 +353,11 @@ diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews
   int max_seg = nseg;
   for (int off = 16; off > 0; off >>= 1) max_seg = max(max_seg, __shfl_xor_sync(0xffffffffu, max_seg, off));
   float Rr = 0.f, Rg = 0.f, Rb = 0.f, Ra = 0.f;  // suffix composite behind the sample
-  int64_t cur = -1;
+  I cur = -1;
   float g8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   int li = -1;  // LUT interval of the register sums lg
   float lg[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  const int64_t vcache = p.v_offset + ray;
+  const float *scalars = ws + p.v_offset + ray;   // sample k's at k * n_rays
   float T[kDiffK];
   for (int sidx = max_seg - 1; sidx >= 0; --sidx) {
     const int k0 = sidx * kDiffK, k1 = sidx < nseg ? min(k0 + kDiffK, n) : k0;
@@ -336,10 +366,14 @@ diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews
     // are loaded kSub at a time so that their latencies overlap
     if (k1 > k0) {
       float Tr = ws[ray * p.n_seg + sidx];
+      const float *at = scalars + (int64_t)k0 * p.n_rays;
       for (int kq = k0; kq < k1; kq += kSub) {
         float vv[kSub];
 #pragma unroll
-        for (int j = 0; j < kSub; ++j) vv[j] = kq + j < k1 ? ws[vcache + (int64_t)(kq + j) * p.n_rays] : 0.f;
+        for (int j = 0; j < kSub; ++j) {
+          vv[j] = kq + j < k1 ? *at : 0.f;
+          at += p.n_rays;
+        }
 #pragma unroll
         for (int j = 0; j < kSub; ++j) {
           T[kq - k0 + j] = Tr;
@@ -352,24 +386,27 @@ diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews
     // the next sample are loaded one step ahead
     {
       const int jn = (int)__reduce_max_sync(0xffffffffu, (unsigned)(k1 - k0));
-      float v_next = k1 > k0 + jn - 1 ? ws[vcache + (int64_t)(k0 + jn - 1) * p.n_rays] : 0.f;
+      const float *at = scalars + (int64_t)(k0 + jn - 1) * p.n_rays;
+      float v_next = k1 > k0 + jn - 1 ? *at : 0.f;
       float t_next = T[max(jn - 1, 0)];
       for (int j = jn - 1; j >= 0; --j) {
         const int k = k0 + j;
         const bool on = k < k1;
         const float v_cur = v_next, Tk = t_next;
         if (j > 0) {
-          v_next = k - 1 < k1 ? ws[vcache + (int64_t)(k - 1) * p.n_rays] : 0.f;
+          at -= p.n_rays;
+          v_next = k - 1 < k1 ? *at : 0.f;
           t_next = T[j - 1];
         }
-        int64_t base = -1;
+        I base = -1;
         float w[3] = {0.f, 0.f, 0.f}, dv = 0.f;
         if (on) {
           const float t = fmaf((float)k, p.sample_dist, t0);
-          base = diff_cell(g, A, B, t, w);
+          base = diff_cell<I>(g, A, B, t, w);
           float s_raw, wl;
           int i0;
-          const float4 c = diff_lut(lut, p, v_cur, s_raw, i0, wl);
+          float4 st;   // d(rgba)/dx, x = s (n - 1)
+          const float4 c = diff_lut(lut, p, v_cur, s_raw, i0, wl, st);
           const float ta = Tk * c.w;
           const float dcr = ta * gr.x, dcg = ta * gr.y, dcb = ta * gr.z;
           const float da = Tk * (gr.x * (c.x - Rr) + gr.y * (c.y - Rg) + gr.z * (c.z - Rb) +
@@ -393,37 +430,31 @@ diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews
           lg[5] = fmaf(wl, dcg, lg[5]);
           lg[6] = fmaf(wl, dcb, lg[6]);
           lg[7] = fmaf(wl, da, lg[7]);
-          // scalar: d(rgba)/dx = lut[i0 + 1] - lut[i0], x = s (n - 1)
-          if (s_raw > 0.f && s_raw < 1.f) {
-            const float4 a0 = lut[i0], a1 = lut[i0 + 1];
-            const float dx = dcr * (a1.x - a0.x) + dcg * (a1.y - a0.y) + dcb * (a1.z - a0.z) +
-                             da * (a1.w - a0.w);
-            dv = dx * (float)(p.lut_size - 1) * p.inv_range;
-          }
+          if (s_raw > 0.f && s_raw < 1.f)
+            dv = (dcr * st.x + dcg * st.y + dcb * st.z + da * st.w) * (float)(p.lut_size - 1) * p.inv_range;
         }
         // pool the field gradient per cell; flush when a lane changes cell
         const bool change = on && base != cur && cur >= 0;
-        flush_cell(gq, g, cur, g8, change);
+        flush_cell<I>(gq, g, cur, g8, change);
         if (change) {
 #pragma unroll
           for (int m = 0; m < 8; ++m) g8[m] = 0.f;
         }
         if (on) {
           cur = base;
-          const float x0 = 1.f - w[0], y0 = 1.f - w[1], z0 = 1.f - w[2];
-          g8[0] = fmaf(dv, x0 * y0 * z0, g8[0]);
-          g8[1] = fmaf(dv, w[0] * y0 * z0, g8[1]);
-          g8[2] = fmaf(dv, x0 * w[1] * z0, g8[2]);
-          g8[3] = fmaf(dv, w[0] * w[1] * z0, g8[3]);
-          g8[4] = fmaf(dv, x0 * y0 * w[2], g8[4]);
-          g8[5] = fmaf(dv, w[0] * y0 * w[2], g8[5]);
-          g8[6] = fmaf(dv, x0 * w[1] * w[2], g8[6]);
-          g8[7] = fmaf(dv, w[0] * w[1] * w[2], g8[7]);
+          const float x0 = 1.f - w[0], y0 = 1.f - w[1];
+          const float lo = dv * (1.f - w[2]), hi = dv * w[2];
+          const float xy[4] = {x0 * y0, w[0] * y0, x0 * w[1], w[0] * w[1]};
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            g8[m] = fmaf(lo, xy[m], g8[m]);
+            g8[4 + m] = fmaf(hi, xy[m], g8[4 + m]);
+          }
         }
       }
     }
   }
-  flush_cell(gq, g, cur, g8, cur >= 0);
+  flush_cell<I>(gq, g, cur, g8, cur >= 0);
   flush_lut4(slg, li, lg);
 }
 
@@ -475,6 +506,7 @@ int diff_setup(const float *field, const int dims[3], const double origin[3],
   p.n_seg = (int)((max_samples + kDiffK - 1) / kDiffK);
   p.lut_copies = 1;
   p.n_rays = (int64_t)n_views * params->width * params->height;
+  p.packets = params->width % 8 == 0 && params->height % 4 == 0;
   p.v_offset = p.n_rays * p.n_seg;
   return GVR_OK;
 }
@@ -511,11 +543,13 @@ int gvr_diff_render_forward(const float *field, const int dims[3], const double 
   if (rc != GVR_OK) return rc;
   if (!lut || !rgba) return set_error(GVR_ERR_INVALID_ARGUMENT, "NULL lut or rgba");
   const size_t smem = sizeof(float4) * p.lut_size;
-  cudaError_t e = cudaFuncSetAttribute(diff_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const bool small = (int64_t)dims[0] * dims[1] * dims[2] < ((int64_t)1 << 31);
+  const auto forward = small ? diff_forward<int> : diff_forward<int64_t>;
+  cudaError_t e = cudaFuncSetAttribute(forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(sizeof(float4) * kDiffLut));
   if (e != cudaSuccess) return cuda_error(e, "shared-memory attribute");
   dim3 grid((p.width + 15) / 16, (p.height + 15) / 16, n_views);
-  diff_forward<<<grid, 256, smem, (cudaStream_t)stream>>>(field, g, views, p, (const float4 *)lut,
+  forward<<<grid, 256, smem, (cudaStream_t)stream>>>(field, g, views, p, (const float4 *)lut,
                                                           (float4 *)rgba, workspace);
   count_launch();
   e = cudaGetLastError();
@@ -537,7 +571,9 @@ int gvr_diff_render_backward(const float *field, const int dims[3], const double
   if (!lut || !grad_rgba || !workspace || !grad_field || !grad_lut)
     return set_error(GVR_ERR_INVALID_ARGUMENT, "NULL buffer");
   const size_t smem = (sizeof(float4) + sizeof(float)) * p.lut_size;
-  cudaError_t e = cudaFuncSetAttribute(diff_backward, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const bool small = (int64_t)dims[0] * dims[1] * dims[2] < ((int64_t)1 << 31);
+  const auto backward = small ? diff_backward<int> : diff_backward<int64_t>;
+  cudaError_t e = cudaFuncSetAttribute(backward, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return cuda_error(e, "shared-memory attribute");
   // corner-quad buffer of the field gradient, from the library's pool
@@ -556,7 +592,7 @@ int gvr_diff_render_backward(const float *field, const int dims[3], const double
   if (e == cudaSuccess) e = cudaMemsetAsync(glc, 0, sizeof(float) * 4 * p.lut_size * p.lut_copies, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(gq, 0, sizeof(float4) * nodes, st);
   if (e == cudaSuccess) {
-    diff_backward<<<grid, 256, smem, st>>>(field, g, views, p, (const float4 *)lut,
+    backward<<<grid, 256, smem, st>>>(field, g, views, p, (const float4 *)lut,
                                            (const float4 *)grad_rgba, workspace, gq, glc);
     count_launch();
     sum_lut_copies<<<dim3((4 * p.lut_size + 255) / 256, (unsigned)((p.lut_copies + 31) / 32)), 256, 0,
