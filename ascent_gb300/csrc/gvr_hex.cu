@@ -153,10 +153,11 @@ __device__ __forceinline__ int prefix(const uint32_t *codes, int n_leaves, int a
   return 32 + __clz((uint32_t)a ^ (uint32_t)b);
 }
 
-// One thread per inner node i in [0, n_leaves - 2]: children and parents.
+// One thread per inner node i in [0, n_leaves - 2]: children, parents, and the
+// leaves below it.
 __global__ void karras_kernel(const uint32_t *__restrict__ codes, int n_leaves,
                               int *__restrict__ left, int *__restrict__ right,
-                              int *__restrict__ parent)
+                              int *__restrict__ parent, int4 *__restrict__ range)
 {
   const int n_inner = n_leaves - 1;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_inner; i += gridDim.x * blockDim.x) {
@@ -181,74 +182,114 @@ __global__ void karras_kernel(const uint32_t *__restrict__ codes, int n_leaves,
     const int rc = hi == split + 1 ? n_inner + split + 1 : split + 1;
     left[i] = lc;
     right[i] = rc;
+    range[i] = make_int4(lo, hi, split, 0);
     parent[lc] = i;
     parent[rc] = i;
     if (i == 0) parent[0] = -1;
   }
 }
 
-// Bottom-up refit: the second thread to reach a node computes its box.
-__global__ void refit_kernel(const float4 *__restrict__ leaf_lo, const float4 *__restrict__ leaf_hi,
-                             const uint32_t *__restrict__ ids, int n_leaves,
-                             const int *__restrict__ left, const int *__restrict__ right,
-                             const int *__restrict__ parent, int *__restrict__ counters,
-                             float4 *box)
+// Bottom-up refit, and the flat layout of each node as its box is made: the
+// second thread to reach a node joins its children's boxes. Nodes whose leaves
+// all belong to one CTA's 256 (all but some 2 in 256) are joined in shared
+// memory, with no fence wider than the CTA; the others through global memory
+// with an arrival counter each, a serial chain of fences up to the root. With
+// every node through global memory 125 us for 1M cells and 27 for the layout
+// pass after it; 114 us so for both.
+constexpr int kRefitLeaves = 256;
+
+__device__ __forceinline__ void join(const float4 l[2], const float4 h[2], float4 &lo, float4 &hi)
 {
-  const int n_inner = n_leaves - 1;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n_leaves; k += gridDim.x * blockDim.x) {
-    int node = parent[n_inner + k];
-    while (node >= 0) {
-      __threadfence();
-      if (atomicAdd(&counters[node], 1) == 0) break;
-      __threadfence();
-      float4 l[2], h[2];
-      const int ch[2] = {left[node], right[node]};
-      for (int q = 0; q < 2; ++q) {
-        if (ch[q] >= n_inner) {
-          const uint32_t cell = ids[ch[q] - n_inner];
-          l[q] = leaf_lo[cell];
-          h[q] = leaf_hi[cell];
-        } else {
-          l[q] = __ldcg(box + 2 * ch[q]);
-          h[q] = __ldcg(box + 2 * ch[q] + 1);
-        }
-      }
-      box[2 * node] = make_float4(fminf(l[0].x, l[1].x), fminf(l[0].y, l[1].y),
-                                  fminf(l[0].z, l[1].z), 0.f);
-      box[2 * node + 1] = make_float4(fmaxf(h[0].x, h[1].x), fmaxf(h[0].y, h[1].y),
-                                      fmaxf(h[0].z, h[1].z), 0.f);
-      node = parent[node];
-    }
-  }
+  lo = make_float4(fminf(l[0].x, l[1].x), fminf(l[0].y, l[1].y), fminf(l[0].z, l[1].z), 0.f);
+  hi = make_float4(fmaxf(h[0].x, h[1].x), fmaxf(h[0].y, h[1].y), fmaxf(h[0].z, h[1].z), 0.f);
 }
 
-__global__ void emit_kernel(const float4 *__restrict__ leaf_lo, const float4 *__restrict__ leaf_hi,
-                            const uint32_t *__restrict__ ids, int n_leaves,
-                            const int *__restrict__ left, const int *__restrict__ right,
-                            const float4 *__restrict__ box, float4 *__restrict__ bvh)
+// The flat node (see gvr_hex_device.cuh) from its children and their boxes.
+__device__ __forceinline__ void write_node(float4 *__restrict__ bvh, int node, const int ch[2], int n_inner,
+                                           const float4 l[2], const float4 h[2])
 {
+  const int e0 = ch[0] >= n_inner ? -(ch[0] - n_inner + 1) : ch[0];
+  const int e1 = ch[1] >= n_inner ? -(ch[1] - n_inner + 1) : ch[1];
+  float4 *q = bvh + 4 * (int64_t)node;
+  q[0] = make_float4(l[0].x, l[0].y, l[0].z, h[0].x);
+  q[1] = make_float4(h[0].y, h[0].z, l[1].x, l[1].y);
+  q[2] = make_float4(l[1].z, h[1].x, h[1].y, h[1].z);
+  q[3] = make_float4(__int_as_float(e0), __int_as_float(e1), 0.f, 0.f);
+}
+
+__global__ void __launch_bounds__(kRefitLeaves)
+refit_kernel(const float4 *__restrict__ leaf_lo, const float4 *__restrict__ leaf_hi,
+             const uint32_t *__restrict__ ids, int n_leaves, const int *__restrict__ parent,
+             const int4 *__restrict__ range, int *__restrict__ counters, float4 *box, float4 *__restrict__ bvh)
+{
+  // boxes of the CTA's leaves, then of its inner nodes (one per leaf number)
+  __shared__ float4 s_lo[2 * kRefitLeaves], s_hi[2 * kRefitLeaves];
+  __shared__ int s_seen[kRefitLeaves];
   const int n_inner = n_leaves - 1;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_inner; i += gridDim.x * blockDim.x) {
-    float4 l[2], h[2];
-    int enc[2];
-    const int ch[2] = {left[i], right[i]};
+  const int b0 = blockIdx.x * kRefitLeaves, k = b0 + threadIdx.x;
+  int node = -1;
+  if (k < n_leaves) {
+    const uint32_t cell = ids[k];
+    s_lo[threadIdx.x] = leaf_lo[cell];
+    s_hi[threadIdx.x] = leaf_hi[cell];
+    node = parent[n_inner + k];
+  }
+  s_seen[threadIdx.x] = 0;
+  __syncthreads();
+  // a node's leaves and split tell its children: one load a level, the parent's
+  // along with it
+  auto child = [&](const int4 &r, int q) {
+    return q == 0 ? (r.x == r.z ? n_inner + r.z : r.z) : (r.y == r.z + 1 ? n_inner + r.z + 1 : r.z + 1);
+  };
+  while (node >= 0) {
+    const int4 r = range[node];
+    const int up = parent[node];
+    if (r.x < b0 || r.y >= b0 + kRefitLeaves) break;
+    // the node's number is one of its own leaves', so it is in the CTA's range
+    __threadfence_block();
+    if (atomicAdd(&s_seen[node - b0], 1) == 0) {
+      node = -1;
+      break;
+    }
+    __threadfence_block();
+    const int ch[2] = {child(r, 0), child(r, 1)};
+    float4 l[2], h[2], lo, hi;
+    for (int q = 0; q < 2; ++q) {
+      const int at = ch[q] >= n_inner ? ch[q] - n_inner - b0 : kRefitLeaves + ch[q] - b0;
+      l[q] = s_lo[at];
+      h[q] = s_hi[at];
+    }
+    join(l, h, lo, hi);
+    s_lo[kRefitLeaves + node - b0] = lo;
+    s_hi[kRefitLeaves + node - b0] = hi;
+    box[2 * (int64_t)node] = lo;
+    box[2 * (int64_t)node + 1] = hi;
+    write_node(bvh, node, ch, n_inner, l, h);
+    node = up;
+  }
+  while (node >= 0) {
+    const int4 r = range[node];
+    const int up = parent[node];
+    __threadfence();
+    if (atomicAdd(&counters[node], 1) == 0) break;
+    __threadfence();
+    const int ch[2] = {child(r, 0), child(r, 1)};
+    float4 l[2], h[2], lo, hi;
     for (int q = 0; q < 2; ++q) {
       if (ch[q] >= n_inner) {
-        const int k = ch[q] - n_inner;
-        const uint32_t cell = ids[k];
+        const uint32_t cell = ids[ch[q] - n_inner];
         l[q] = leaf_lo[cell];
         h[q] = leaf_hi[cell];
-        enc[q] = -(k + 1);
       } else {
-        l[q] = box[2 * ch[q]];
-        h[q] = box[2 * ch[q] + 1];
-        enc[q] = ch[q];
+        l[q] = __ldcg(box + 2 * (int64_t)ch[q]);
+        h[q] = __ldcg(box + 2 * (int64_t)ch[q] + 1);
       }
     }
-    bvh[4 * (int64_t)i + 0] = make_float4(l[0].x, l[0].y, l[0].z, h[0].x);
-    bvh[4 * (int64_t)i + 1] = make_float4(h[0].y, h[0].z, l[1].x, l[1].y);
-    bvh[4 * (int64_t)i + 2] = make_float4(l[1].z, h[1].x, h[1].y, h[1].z);
-    bvh[4 * (int64_t)i + 3] = make_float4(__int_as_float(enc[0]), __int_as_float(enc[1]), 0.f, 0.f);
+    join(l, h, lo, hi);
+    box[2 * (int64_t)node] = lo;
+    box[2 * (int64_t)node + 1] = hi;
+    write_node(bvh, node, ch, n_inner, l, h);
+    node = up;
   }
 }
 
@@ -378,18 +419,31 @@ __device__ __forceinline__ void face_triple(const int4 *__restrict__ conn, uint3
 constexpr unsigned kFaceBucket = 256;
 
 // cnt[n] += faces whose smallest node is n; slot[f]: face f's place in its
-// bucket.
+// bucket. A thread per cell, whose six atomics are in flight together (a thread
+// per face, as in the two passes after it, took 31 against 16 us for 1M cells).
 __global__ void __launch_bounds__(256)
-face_count_kernel(const int4 *__restrict__ conn, int64_t nf, uint32_t *__restrict__ cnt,
+face_count_kernel(const int4 *__restrict__ conn, int64_t n_cells, uint32_t *__restrict__ cnt,
                   uint32_t *__restrict__ slot, int *__restrict__ crowded)
 {
-  for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < nf;
-       f += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t t[3];
-    face_triple(conn, (uint32_t)f, t);
-    const uint32_t s = atomicAdd(cnt + t[0], 1u);
-    slot[f] = s;
-    if (s >= kFaceBucket) *crowded = 1;
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n_cells;
+       c += (int64_t)gridDim.x * blockDim.x) {
+    const int4 a = conn[2 * c], b = conn[2 * c + 1];
+    // each face's smallest node, numbered like kHexFace
+    const uint32_t x = min((uint32_t)a.x, (uint32_t)a.y), y = min((uint32_t)a.z, (uint32_t)a.w);
+    const uint32_t z = min((uint32_t)b.x, (uint32_t)b.y), w = min((uint32_t)b.z, (uint32_t)b.w);
+    const uint32_t low[6] = {min(min((uint32_t)a.x, (uint32_t)a.w), min((uint32_t)b.x, (uint32_t)b.w)),
+                             min(min((uint32_t)a.y, (uint32_t)a.z), min((uint32_t)b.y, (uint32_t)b.z)),
+                             min(x, z), min(y, w), min(x, y), min(z, w)};
+    uint32_t s[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) s[k] = atomicAdd(cnt + low[k], 1u);
+    bool full = false;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      slot[6 * c + k] = s[k];
+      full = full || s[k] >= kFaceBucket;
+    }
+    if (full) *crowded = 1;
   }
 }
 
@@ -659,7 +713,7 @@ static int build_neighbours(Domain &d)
   NB_TRY(dev_alloc(&d_crowded, 1), "alloc flag");
   NB_TRY(cudaMemsetAsync(d_crowded, 0, sizeof(int), 0), "clear flag");
   NB_TRY(cudaMemsetAsync(off, 0, sizeof(uint32_t) * (nn + 1), 0), "clear face buckets");
-  face_count_kernel<<<grid_for(nf), 256>>>(d.d_conn, nf, off, slot, d_crowded);
+  face_count_kernel<<<grid_for(d.n_cells), 256>>>(d.d_conn, d.n_cells, off, slot, d_crowded);
   count_launch();
   NB_TRY(exclusive_scan(off, nn + 1, scan_tmp, 0), "scan face buckets");
   face_fill_kernel<<<grid_for(nf), 256>>>(d.d_conn, nf, off, slot, bucket, d_crowded);
@@ -693,6 +747,7 @@ static int build_hex(Domain &d, const void *x, const void *y, const void *z, int
   float *part = nullptr;
   uint32_t *keys_tmp = nullptr, *vals_tmp = nullptr, *sort_scr = nullptr;
   int *counters = nullptr;
+  int4 *range = nullptr;
   int rc = GVR_OK;
   cudaError_t e = cudaSuccess;
   const auto t0 = std::chrono::steady_clock::now();
@@ -776,14 +831,11 @@ static int build_hex(Domain &d, const void *x, const void *y, const void *z, int
       HEX_TRY(dev_alloc(&counters, ni), "alloc counters");
       HEX_TRY(dev_alloc(&d.d_bvh, 4 * ni), "alloc bvh");
       HEX_TRY(cudaMemset(counters, 0, sizeof(int) * ni), "clear counters");
-      karras_kernel<<<grid_for(ni), 256>>>(d.d_codes, (int)nc, d.d_left, d.d_right, d.d_parent);
-      count_launch();
-      refit_kernel<<<grid_for(nc), 256>>>(leaf_lo, leaf_hi, d.d_ids, (int)nc, d.d_left, d.d_right,
-                                          d.d_parent, counters, d.d_inner_box);
-      count_launch();
-      emit_kernel<<<grid_for(ni), 256>>>(leaf_lo, leaf_hi, d.d_ids, (int)nc, d.d_left, d.d_right,
-                                         d.d_inner_box, d.d_bvh);
-      count_launch();
+      HEX_TRY(dev_alloc(&range, ni), "alloc tree");
+      karras_kernel<<<grid_for(ni), 256>>>(d.d_codes, (int)nc, d.d_left, d.d_right, d.d_parent, range);
+      refit_kernel<<<(unsigned)((nc + kRefitLeaves - 1) / kRefitLeaves), kRefitLeaves>>>(
+          leaf_lo, leaf_hi, d.d_ids, (int)nc, d.d_parent, range, counters, d.d_inner_box, d.d_bvh);
+      count_launch(2);
     }
     HEX_TRY(cudaGetLastError(), "BVH build launch");
     HEX_TRY(cudaDeviceSynchronize(), "BVH build");
@@ -804,6 +856,7 @@ done:
   device_free_idle(vals_tmp);
   device_free_idle(sort_scr);
   device_free_idle(counters);
+  device_free_idle(range);
   d.bvh_build_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
   if (rc == GVR_OK) rc = build_neighbours(d);
   d.dev.hex_nbr = d.d_nbr;

@@ -69,3 +69,34 @@ def test_crowded_node(cells):
     pts = rng.uniform(0, 1, (60, 3))
     conn = np.stack([np.concatenate([[0], 1 + rng.permutation(59)[:7]]) for _ in range(cells)]).astype(np.int32)
     check(pts, conn)
+
+
+@pytest.mark.parametrize("cells", [2, 3, 255, 256, 257, 511, 1000, 3000])
+def test_refit(cells):
+    """The tree's boxes, whose nodes are joined in shared memory where their
+    leaves belong to one block of 256, against boxes joined from the leaves up
+    in numpy; and every point at a cell's middle is found through them."""
+    rng = np.random.default_rng(cells)
+    pts, conn = grid(int(np.ceil(cells ** (1 / 3))), rng, True)
+    conn = np.ascontiguousarray(conn[:cells])
+    x, y, z = (np.ascontiguousarray(pts[:, a], dtype=np.float32) for a in range(3))
+    with S.Scene(0) as sc:
+        did = sc.add_hex(x, y, z, conn, x)
+        t = sc.hex_bvh(did)
+        mid = np.stack([v[conn].mean(axis=1) for v in (x, y, z)], 1)
+        found, _ = sc.hex_locate(did, mid)
+    np.testing.assert_array_equal(found, np.arange(cells))
+    xyz = np.stack([x, y, z], 1)
+    n_inner = cells - 1
+    box = np.zeros((2 * cells - 1, 6), np.float32)
+    box[n_inner:, :3] = xyz[conn[t["ids"]]].min(axis=1)
+    box[n_inner:, 3:] = xyz[conn[t["ids"]]].max(axis=1)
+    done = np.zeros(2 * cells - 1, bool)
+    done[n_inner:] = True
+    while not done.all():
+        for i in np.nonzero(~done)[0]:
+            l, r = t["left"][i], t["right"][i]
+            if done[l] and done[r]:
+                box[i, :3], box[i, 3:] = np.minimum(box[l, :3], box[r, :3]), np.maximum(box[l, 3:], box[r, 3:])
+                done[i] = True
+    np.testing.assert_array_equal(t["inner_box"][:n_inner], box[:n_inner])
