@@ -48,7 +48,8 @@ def build(force: bool = False, extra: list[str] | None = None) -> Path:
     """Compile csrc/ into libgvr.so; skip when the library is newer than every source."""
     extra = list(extra or [])
     srcs = sources()
-    deps = srcs + sorted(CSRC.glob("*.h")) + [PKG.parent / "include" / "gvr.h", Path(__file__)]
+    headers = sorted(CSRC.glob("*.h")) + sorted(CSRC.glob("*.cuh"))
+    deps = srcs + headers + [PKG.parent / "include" / "gvr.h", Path(__file__)]
     if not force and LIB.exists():
         newest = max(p.stat().st_mtime for p in deps)
         if LIB.stat().st_mtime > newest:

@@ -1,7 +1,7 @@
 // gvr_diff.cu — differentiable volume render: forward with transmittance
 // checkpoints and its hand-written adjoint.
 //
-// The render is the single-uniform-domain march of gvr_march.cu (same ray
+// The render is the single-uniform-domain march of gvr_march_device.cuh (same ray
 // model, stepping rule and front-to-back blend) with the two changes a
 // gradient needs: the transfer function is looked up with linear
 // interpolation (so colour and opacity are differentiable in the scalar),

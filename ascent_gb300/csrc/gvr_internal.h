@@ -344,7 +344,7 @@ cudaError_t launch_march(const DomainDev *d_domains, const ViewDev &view,
 constexpr int kCostOrderTiles = 48 * 1024;
 cudaError_t launch_tile_cost_order(const DomainDev *d_domains, const ViewDev &view, const MarchParams &mp,
                                    int *d_order, unsigned *d_keys, unsigned *d_top, cudaStream_t stream);
-// staged march (gvr_march.cu): uniform vertex-field domains only, taken in
+// staged march (gvr_staged.cu): uniform vertex-field domains only, taken in
 // `order`; *d_stage_fail counts CTAs whose bounded wait for their bulk
 // copies gave up (they finish from global memory)
 cudaError_t launch_staged(const DomainDev *d_domains, const ViewDev &view, const MarchParams &mp,
