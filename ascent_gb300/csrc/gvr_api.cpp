@@ -126,8 +126,9 @@ void device_free_idle(void *ptr)
 void device_free(void *ptr)
 {
   if (!ptr) return;
-  cudaDeviceSynchronize();
-  device_free_idle(ptr);
+  // where the wait is refused (a stream capture in progress) the memory is
+  // left, as cudaFree would leave it: it may still be in use
+  if (cudaDeviceSynchronize() == cudaSuccess) device_free_idle(ptr);
 }
 
 // The device's default memory pool gives its free memory back to the
@@ -534,32 +535,35 @@ int gvr_scene_destroy(gvr_scene *s)
 {
   if (!s) return GVR_OK;
   cudaSetDevice(s->device);
-  cudaDeviceSynchronize();   // whatever still renders from the scene, on any stream
-  for (Domain &d : s->domains) free_domain(d);
-  device_free_idle(s->d_domains);
-  device_free_idle(s->d_lut);
-  device_free_idle(s->d_any_empty);
-  device_free_idle(s->d_counters);
-  device_free_idle(s->d_rgba_tmp);
-  device_free_idle(s->d_depth_tmp);
-  device_free_idle(s->d_views);
-  device_free_idle(s->d_rects);
-  device_free_idle(s->d_queue);
-  for (auto &t : s->tile_orders) device_free_idle(t.second);
-  device_free_idle(s->d_cost_order);
-  device_free_idle(s->d_batch_rgba);
-  device_free_idle(s->d_batch_depth);
+  // whatever still renders from the scene, on any stream; device memory is
+  // left where the wait is refused (see device_free)
+  if (cudaDeviceSynchronize() == cudaSuccess) {
+    for (Domain &d : s->domains) free_domain(d);
+    device_free_idle(s->d_domains);
+    device_free_idle(s->d_lut);
+    device_free_idle(s->d_any_empty);
+    device_free_idle(s->d_counters);
+    device_free_idle(s->d_rgba_tmp);
+    device_free_idle(s->d_depth_tmp);
+    device_free_idle(s->d_views);
+    device_free_idle(s->d_rects);
+    device_free_idle(s->d_queue);
+    for (auto &t : s->tile_orders) device_free_idle(t.second);
+    device_free_idle(s->d_cost_order);
+    device_free_idle(s->d_batch_rgba);
+    device_free_idle(s->d_batch_depth);
+    for (void *b : s->stage) device_free_idle(b);
+    device_free_idle(s->d_ranges);
+    device_free_idle(s->d_flag);
+  }
   if (s->batch_exec) cudaGraphExecDestroy(s->batch_exec);
   if (s->own_stream) cudaStreamDestroy(s->own_stream);
   if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
   for (int b = 0; b < gvr_scene::kStageMax; ++b) {
-    device_free_idle(s->stage[b]);
     if (s->copied[b]) cudaEventDestroy(s->copied[b]);
     if (s->consumed[b]) cudaEventDestroy(s->consumed[b]);
   }
-  device_free_idle(s->d_ranges);
   cudaFreeHost(s->h_ranges);
-  device_free_idle(s->d_flag);
   delete s;
   return GVR_OK;
 }

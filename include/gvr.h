@@ -536,8 +536,10 @@ GVR_API int gvr_zbuffer_composite(int n_images, const float *const *rgba,
  * and stays reserved until the process exits or this call trims it), so
  * that repeated calls neither map fresh pages nor synchronise. An in-situ
  * host that needs the memory back between visualisation steps calls this;
- * the next call that needs scratch allocates it again. reserved_out (may be
- * NULL) receives the bytes the pool still reserves. Synchronise the streams
+ * the next call that needs scratch allocates it again. Scenes' memory comes
+ * from a second pool, which keeps at most 4 GiB that no scene uses; this call
+ * trims it to keep_bytes too. reserved_out (may be NULL) receives the bytes
+ * the scratch pool still reserves. Synchronise the streams
  * that used the library before trimming, or their last frees may not have
  * completed yet. */
 GVR_API int gvr_scratch_trim(int device, uint64_t keep_bytes, uint64_t *reserved_out);
