@@ -14,8 +14,8 @@
 // in a workspace ([sample][ray], so that a warp writes contiguous rays).
 // Backward: per ray, segments from last to first. A segment's transmittances
 // T_k are rebuilt forward from its checkpoint through the cached scalars and
-// the LUT — no field loads, and the blend is never inverted — into a
-// thread-local array; then its samples are walked back to front with the
+// the LUT — no field loads, and the blend is never inverted — into an
+// array of the thread's; then its samples are walked back to front with the
 // suffix composite (R', A') of the samples behind them:
 //   dL/dc_k = T_k a_k g_rgb,
 //   dL/da_k = T_k (g_rgb . (c_k - R'_k) + g_A (1 - A'_k)),
@@ -42,6 +42,7 @@ constexpr int kDiffK = 64;          // samples per transmittance checkpoint
 constexpr int kSub = 8;             // backward: scalars loaded together
 constexpr int kMaxDiffViews = 64;
 constexpr int kDiffLut = 4096;
+constexpr int kSharedTLut = 512;    // backward: transmittances in shared memory up to this LUT
 
 struct DiffViews {
   ViewDev v[kMaxDiffViews];
@@ -426,7 +427,13 @@ __device__ __forceinline__ void flush_lut4(float *copy, int li, float (&lg)[8])
   for (int m = 0; m < 8; ++m) lg[m] = 0.f;
 }
 
-template <typename I>
+// A segment's transmittances lie in shared memory where three CTAs per SM still
+// fit with them (SHARED_T: 64 KB and 20 bytes per LUT entry each), else in local
+// memory, which the L1 does not hold (200 KB per SM): 1930 -> 1856 us for a
+// 128^3 field, 16 views at 256^2. What is left is issue (67%) and reductions on
+// their way to L2 (L1-to-crossbar requests 58%); four CTAs per SM at 64
+// registers ran the same.
+template <typename I, bool SHARED_T>
 __global__ void __launch_bounds__(256)
 diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews views,
               const DiffParams p, const float4 *__restrict__ g_lut,
@@ -480,7 +487,9 @@ diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews
   int li = -1;  // LUT interval of the register sums lg
   float lg[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const float *scalars = ws + p.v_offset + ray;   // sample k's at k * n_rays
-  float T[kDiffK];
+  float local_t[SHARED_T ? 1 : kDiffK];
+  float *T = SHARED_T ? lut_a + p.lut_size + threadIdx.x : local_t;   // sample j's at j * kStep
+  constexpr int kStep = SHARED_T ? 256 : 1;
   for (int sidx = max_seg - 1; sidx >= 0; --sidx) {
     const int k0 = sidx * kDiffK, k1 = sidx < nseg ? min(k0 + kDiffK, n) : k0;
     // transmittance of every sample of the segment, forward from its
@@ -498,7 +507,7 @@ diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews
         }
 #pragma unroll
         for (int j = 0; j < kSub; ++j) {
-          T[kq - k0 + j] = Tr;
+          T[kStep * (kq - k0 + j)] = Tr;
           if (kq + j < k1) Tr *= 1.f - lut_alpha(lut_a, p, vv[j]);
         }
       }
@@ -510,7 +519,7 @@ diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews
       const int jn = (int)__reduce_max_sync(0xffffffffu, (unsigned)(k1 - k0));
       const float *at = scalars + (int64_t)(k0 + jn - 1) * p.n_rays;
       float v_next = k1 > k0 + jn - 1 ? *at : 0.f;
-      float t_next = T[max(jn - 1, 0)];
+      float t_next = T[kStep * max(jn - 1, 0)];
       for (int j = jn - 1; j >= 0; --j) {
         const int k = k0 + j;
         const bool on = k < k1;
@@ -518,7 +527,7 @@ diff_backward(const float *__restrict__ field, const DiffGrid g, const DiffViews
         if (j > 0) {
           at -= p.n_rays;
           v_next = k - 1 < k1 ? *at : 0.f;
-          t_next = T[j - 1];
+          t_next = T[kStep * (j - 1)];
         }
         I base = -1;
         float w[3] = {0.f, 0.f, 0.f}, dv = 0.f;
@@ -760,11 +769,17 @@ int gvr_diff_render_backward(const float *field, const int dims[3], const double
   if (rc != GVR_OK) return rc;
   if (!lut || !grad_rgba || !workspace || !grad_field || !grad_lut)
     return set_error(GVR_ERR_INVALID_ARGUMENT, "NULL buffer");
-  const size_t smem = (sizeof(float4) + sizeof(float)) * p.lut_size;
+  const bool shared_t = p.lut_size <= kSharedTLut;
+  // of n LUT entries; the attribute is set to the kernel's largest, whatever other threads launch
+  const auto shared_bytes = [&](int n) {
+    return (sizeof(float4) + sizeof(float)) * n + (shared_t ? sizeof(float) * 256 * kDiffK : 0);
+  };
+  const size_t smem = shared_bytes(p.lut_size);
   const bool small = (int64_t)dims[0] * dims[1] * dims[2] < ((int64_t)1 << 31);
-  const auto backward = small ? diff_backward<int> : diff_backward<int64_t>;
+  const auto backward = shared_t ? (small ? diff_backward<int, true> : diff_backward<int64_t, true>)
+                                 : (small ? diff_backward<int, false> : diff_backward<int64_t, false>);
   cudaError_t e = cudaFuncSetAttribute(backward, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+                                       (int)shared_bytes(shared_t ? kSharedTLut : kDiffLut));
   if (e != cudaSuccess) return cuda_error(e, "shared-memory attribute");
   // corner-quad buffer of the field gradient, from the library's pool
   cudaStream_t st = (cudaStream_t)stream;
