@@ -1040,14 +1040,15 @@ __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_
 template <int UNROLL, int MODE>
 __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, const ViewDev &view,
                                           const MarchParams &mp, const float4 *lut, int px, int py,
-                                          float4 &out, float &dep, float *g_state, bool any_hidden)
+                                          float4 &out, float &dep, float *g_state, bool any_hidden,
+                                          bool by_domain = false)
 {
   if (MODE != kMarchHex && mask) {
     // domains that are all uniform vertex fields in 8^3-cell bricks, two or
     // more of them or one with empty bricks to pass over: the one-loop walk (a
     // single domain without has no crossing to wait at, and its own loop keeps
     // fewer values live: 1.39 against 1.49 ms on the 513^3 field as one domain)
-    bool walk = doms[__ffsll((long long)mask) - 1].bshift == 3 && ((mask & (mask - 1)) != 0 || any_hidden);
+    bool walk = !by_domain && doms[__ffsll((long long)mask) - 1].bshift == 3 && ((mask & (mask - 1)) != 0 || any_hidden);
     if (MODE != kMarchUniform)
       for (uint64_t m = mask; m; m &= m - 1) {
         const DomainDev &dm = doms[__ffsll((long long)m) - 1];
@@ -1126,8 +1127,8 @@ __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, 
                : dm.bshift == 2 ? march_uniform<UNROLL, 2, false>(dm, r, bt0, bt1, mp, lut, thr, acc)
                                 : march_uniform<UNROLL, 4, false>(dm, r, bt0, bt1, mp, lut, thr, acc);
     } else if (uniform_vertex) {
-      // 8^3-cell bricks come here only next to other kinds of domains
-      count += MODE != kMarchUniform && dm.bshift == 3 ? march_bricks<UNROLL, 3>(dm, r, bt0, bt1, mp, lut, thr, acc)
+      // 8^3-cell bricks come here next to other kinds of domains and by_domain
+      count += (MODE != kMarchUniform || by_domain) && dm.bshift == 3 ? march_bricks<UNROLL, 3>(dm, r, bt0, bt1, mp, lut, thr, acc)
              : dm.bshift == 2                          ? march_bricks<UNROLL, 2>(dm, r, bt0, bt1, mp, lut, thr, acc)
                                                        : march_bricks<UNROLL, 4>(dm, r, bt0, bt1, mp, lut, thr, acc);
     }
