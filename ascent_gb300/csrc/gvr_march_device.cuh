@@ -295,8 +295,8 @@ __device__ __noinline__ Partial march_cells(const DomainDev &dm, const Ray r, fl
     B[a] = r.d[a] * dm.inv_spacing[a];
   }
   const int cmax[3] = {dm.dims[0] - 2, dm.dims[1] - 2, dm.dims[2] - 2};
-  const int sy = dm.dims[0] - 1;
-  const int64_t sz = (int64_t)sy * (dm.dims[1] - 1);
+  // a cell-centred field has no limit on its cells, so a z layer may hold 2^31 and more
+  const int64_t sy = dm.dims[0] - 1, sz = sy * (dm.dims[1] - 1);
   const float *__restrict__ cells = dm.cells;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), col = acc;
   int64_t last = -1;
