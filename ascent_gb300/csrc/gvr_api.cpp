@@ -10,7 +10,6 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -40,147 +39,7 @@ int cuda_error(cudaError_t e, const char *what)
   return set_error(code, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-namespace {
-constexpr int kMaxPoolDevices = 64;
-std::mutex g_pool_mu;
-cudaMemPool_t g_pools[kMaxPoolDevices] = {};         // call scratch
-cudaMemPool_t g_scene_pools[kMaxPoolDevices] = {};   // scenes' memory
-cudaStream_t g_scene_streams[kMaxPoolDevices] = {};  // its allocations and frees
-
-// Free memory that a device's scene pool holds on to between scenes.
-constexpr uint64_t kScenePoolKeep = (uint64_t)4 << 30;
-
-// A pool of this library on `device` that keeps up to `keep` free bytes.
-cudaError_t make_pool(int device, uint64_t keep, cudaMemPool_t *out)
-{
-  cudaMemPoolProps props{};
-  props.allocType = cudaMemAllocationTypePinned;
-  props.location.type = cudaMemLocationTypeDevice;
-  props.location.id = device;
-  cudaMemPool_t created = nullptr;
-  cudaError_t e = cudaMemPoolCreate(&created, &props);
-  if (e != cudaSuccess) return e;
-  if ((e = cudaMemPoolSetAttribute(created, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
-    cudaMemPoolDestroy(created);
-    return e;
-  }
-  *out = created;
-  return cudaSuccess;
-}
-}  // namespace
-
-// Scenes' memory. An in-situ host makes a scene per publish, some 30 buffers
-// that cudaMalloc maps and cudaFree unmaps, each call a synchronisation: 3.9
-// of the 6.7 ms of a step with 1M new hexahedra, 1.2 of 3.4 ms of one with
-// four structured host domains. From a pool they cost a microsecond each; the
-// pool gives back what it holds beyond kScenePoolKeep at the next
-// synchronisation, all of it to gvr_scratch_trim, and when an allocation does
-// not fit. Allocations and frees are made on one stream of the pool's own on
-// which nothing runs, and an allocation is waited for, so that the memory may
-// be used on any stream and from any thread.
-cudaError_t device_alloc(void **ptr, size_t bytes)
-{
-  *ptr = nullptr;
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
-  if (e != cudaSuccess) return e;
-  if (device < 0 || device >= kMaxPoolDevices) return cudaMalloc(ptr, bytes);
-  cudaMemPool_t pool;
-  cudaStream_t stream;
-  {
-    std::lock_guard<std::mutex> lock(g_pool_mu);
-    if (!g_scene_streams[device] &&
-        (e = cudaStreamCreateWithFlags(&g_scene_streams[device], cudaStreamNonBlocking)) != cudaSuccess)
-      return e;
-    if (!g_scene_pools[device] && (e = make_pool(device, kScenePoolKeep, &g_scene_pools[device])) != cudaSuccess)
-      return e;
-    pool = g_scene_pools[device];
-    stream = g_scene_streams[device];
-  }
-  e = cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
-  if (e == cudaErrorMemoryAllocation) {
-    // what the pools hold free may be what is missing
-    cudaGetLastError();
-    gvr_scratch_trim(device, 0, nullptr);
-    e = cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
-  }
-  return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
-}
-
-void device_free_idle(void *ptr)
-{
-  if (!ptr) return;
-  int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxPoolDevices) {
-    cudaFree(ptr);
-    return;
-  }
-  cudaStream_t stream;
-  {
-    std::lock_guard<std::mutex> lock(g_pool_mu);
-    stream = g_scene_streams[device];
-  }
-  cudaFreeAsync(ptr, stream);
-}
-
-void device_free(void *ptr)
-{
-  if (!ptr) return;
-  // where the wait is refused (a stream capture in progress) the memory is
-  // left, as cudaFree would leave it: it may still be in use
-  if (cudaDeviceSynchronize() == cudaSuccess) device_free_idle(ptr);
-}
-
-// The device's default memory pool gives its free memory back to the
-// system at every synchronisation (release threshold 0), so a call that
-// allocates tens of MB of scratch and synchronises would map fresh pages
-// every time. This library's own pool keeps what it has allocated (up to
-// its high-water mark, held until the process exits) and leaves the
-// default pool, which other libraries in the process may use, as it is.
-cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream)
-{
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
-  if (e != cudaSuccess) return e;
-  if (device < 0 || device >= kMaxPoolDevices) return cudaMallocAsync(ptr, bytes, stream);
-  cudaMemPool_t pool;
-  {
-    std::lock_guard<std::mutex> lock(g_pool_mu);
-    if (!g_pools[device] && (e = make_pool(device, UINT64_MAX, &g_pools[device])) != cudaSuccess) return e;
-    pool = g_pools[device];
-  }
-  return cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
-}
-
 }  // namespace gvr
-
-int gvr_scratch_trim(int device, uint64_t keep_bytes, uint64_t *reserved_out)
-{
-  using namespace gvr;
-  if (device < 0) return set_error(GVR_ERR_INVALID_ARGUMENT, "negative device");
-  cudaMemPool_t pool = nullptr, scenes = nullptr;
-  if (device < kMaxPoolDevices) {
-    std::lock_guard<std::mutex> lock(g_pool_mu);
-    pool = g_pools[device];
-    scenes = g_scene_pools[device];
-  }
-  uint64_t reserved = 0;
-  // what scenes that are gone have left in their pool; what scenes use stays
-  if (scenes) {
-    const cudaError_t e = cudaMemPoolTrimTo(scenes, (size_t)keep_bytes);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMemPoolTrimTo");
-  }
-  if (pool) {
-    // blocks still in use are kept whatever keep_bytes says; memory freed
-    // on a stream is returned once that free has completed
-    cudaError_t e = cudaMemPoolTrimTo(pool, (size_t)keep_bytes);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMemPoolTrimTo");
-    e = cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
-    if (e != cudaSuccess) return cuda_error(e, "cudaMemPoolGetAttribute");
-  }
-  if (reserved_out) *reserved_out = reserved;
-  return GVR_OK;
-}
 
 namespace gvr {
 namespace {
@@ -531,31 +390,31 @@ static void free_domain(Domain &d)
   d = Domain();
 }
 
+// A domain's device buffers.
+static void domain_memory(const Domain &d, std::vector<void *> &out)
+{
+  for (void *p : {(void *)d.d_bricks, (void *)d.d_cells, (void *)d.d_cell_rec, (void *)d.d_brick_range,
+                  (void *)d.d_brick_empty, d.stg.buf, (void *)d.stg.block_range, (void *)d.d_nodes, (void *)d.d_conn,
+                  (void *)d.d_bvh, (void *)d.d_codes, (void *)d.d_ids, (void *)d.d_left, (void *)d.d_right,
+                  (void *)d.d_parent, (void *)d.d_inner_box, (void *)d.d_nbr, (void *)d.d_coef})
+    out.push_back(p);
+}
+
 int gvr_scene_destroy(gvr_scene *s)
 {
   if (!s) return GVR_OK;
   cudaSetDevice(s->device);
-  // whatever still renders from the scene, on any stream; device memory is
-  // left where the wait is refused (see device_free)
-  if (cudaDeviceSynchronize() == cudaSuccess) {
-    for (Domain &d : s->domains) free_domain(d);
-    device_free_idle(s->d_domains);
-    device_free_idle(s->d_lut);
-    device_free_idle(s->d_any_empty);
-    device_free_idle(s->d_counters);
-    device_free_idle(s->d_rgba_tmp);
-    device_free_idle(s->d_depth_tmp);
-    device_free_idle(s->d_views);
-    device_free_idle(s->d_rects);
-    device_free_idle(s->d_queue);
-    for (auto &t : s->tile_orders) device_free_idle(t.second);
-    device_free_idle(s->d_cost_order);
-    device_free_idle(s->d_batch_rgba);
-    device_free_idle(s->d_batch_depth);
-    for (void *b : s->stage) device_free_idle(b);
-    device_free_idle(s->d_ranges);
-    device_free_idle(s->d_flag);
-  }
+  // whatever still renders from the scene, on any stream, is waited for
+  std::vector<void *> memory;
+  for (const Domain &d : s->domains) domain_memory(d, memory);
+  for (void *p : {(void *)s->d_domains, (void *)s->d_lut, (void *)s->d_any_empty, (void *)s->d_counters,
+                  (void *)s->d_rgba_tmp, (void *)s->d_depth_tmp, (void *)s->d_views, (void *)s->d_rects,
+                  (void *)s->d_queue, (void *)s->d_cost_order, (void *)s->d_batch_rgba, (void *)s->d_batch_depth,
+                  (void *)s->d_ranges, (void *)s->d_flag})
+    memory.push_back(p);
+  for (auto &t : s->tile_orders) memory.push_back(t.second);
+  memory.insert(memory.end(), s->stage, s->stage + gvr_scene::kStageMax);
+  device_free(memory.data(), memory.size());
   if (s->batch_exec) cudaGraphExecDestroy(s->batch_exec);
   if (s->own_stream) cudaStreamDestroy(s->own_stream);
   if (s->copy_stream) cudaStreamDestroy(s->copy_stream);

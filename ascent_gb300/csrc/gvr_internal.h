@@ -269,9 +269,13 @@ cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
 
 // Device memory of scenes and of their builds, from a second pool of this
 // library: usable at once on any stream. device_free waits for the device
-// first, as cudaFree does; device_free_idle is for a caller that has.
+// first, as cudaFree does. Where the wait is refused (a capture in progress)
+// the memory may still be in use: it is kept, and freed after a later call's
+// wait; the refusal is returned. device_free_idle is for a caller that has
+// waited.
 cudaError_t device_alloc(void **ptr, size_t bytes);
-void device_free(void *ptr);
+cudaError_t device_free(void *const *ptrs, size_t n);
+inline cudaError_t device_free(void *ptr) { return device_free(&ptr, 1); }
 void device_free_idle(void *ptr);
 
 // kernels launched by this library since it was loaded

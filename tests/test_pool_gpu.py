@@ -1,0 +1,97 @@
+"""Scenes' memory on the device: destroying a scene beside another thread's
+stream capture.
+"""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from ascent_gb300 import _native as N
+from ascent_gb300 import scene as S
+from ascent_gb300 import volume as V
+from ascent_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+GLOBAL, THREAD_LOCAL, RELAXED = 0, 1, 2
+
+
+class Capture:
+    """An (empty) capture of this thread on a stream of its own."""
+
+    def __init__(self, mode):
+        self.cu = C.CDLL("libcuda.so.1")
+        self.stream = C.c_void_p()
+        torch.cuda.current_stream().synchronize()
+        assert self.cu.cuStreamCreate(C.byref(self.stream), 1) == 0
+        assert self.cu.cuStreamBeginCapture_v2(self.stream, mode) == 0
+
+    def end(self):
+        """Whether the capture was left whole."""
+        graph = C.c_void_p()
+        rc = self.cu.cuStreamEndCapture(self.stream, C.byref(graph))
+        if graph:
+            self.cu.cuGraphDestroy(graph)
+        self.cu.cuStreamDestroy_v2(self.stream)
+        return rc == 0
+
+
+def in_thread(fn):
+    out = []
+    t = threading.Thread(target=lambda: out.append(fn()))
+    t.start()
+    t.join()
+    return out[0]
+
+
+def free_bytes():
+    torch.cuda.synchronize()
+    N.scratch_trim(0, 0)
+    return torch.cuda.mem_get_info(0)[0]
+
+
+def make(wl):
+    sc = S.Scene(0)
+    V.load_workload(sc, wl)
+    return sc
+
+
+def two_domains():
+    """More bytes than the blocks a pool takes from the system; rendered and
+    captured once, so that everything that is made at first use is there."""
+    wl = W.plain_small(n=224, width=96, height=80, parts=(2, 1, 1))
+    cam, p = V.workload_camera(wl), V.workload_params(wl)
+    sc = make(wl)
+    sc.render(cam, p)
+    sc.close()
+    assert Capture(THREAD_LOCAL).end()
+    return wl, cam, p, free_bytes()
+
+
+@pytest.mark.parametrize("mode", [THREAD_LOCAL, RELAXED])
+def test_destroy_beside_capture(mode):
+    wl, cam, p, before = two_domains()
+    a, b = make(wl), make(wl)
+    image = a.render(cam, p)[0]
+    cap = Capture(mode)
+    in_thread(a.close)
+    assert cap.end()
+    assert np.array_equal(b.render(cam, p)[0], image)
+    b.close()
+    assert free_bytes() == before
+
+
+def test_destroy_beside_refusing_capture():
+    """A capture in global mode refuses the wait of every thread: the scene's
+    memory is left to a later one and no error stays behind."""
+    wl, cam, p, before = two_domains()
+    a, b = make(wl), make(wl)
+    image = a.render(cam, p)[0]
+    cap = Capture(GLOBAL)
+    in_thread(a.close)
+    cap.end()
+    assert np.array_equal(b.render(cam, p)[0], image)
+    b.close()
+    assert free_bytes() == before
