@@ -200,6 +200,29 @@ void make_view(const gvr_camera &cam, int width, int height, ViewDev *v)
 
 }  // namespace gvr
 
+namespace gvr {
+
+// A domain's device buffers.
+static void domain_memory(const Domain &d, std::vector<void *> &out)
+{
+  for (void *p : {(void *)d.d_bricks, (void *)d.d_cells, (void *)d.d_cell_rec, (void *)d.d_brick_range,
+                  (void *)d.d_brick_empty, d.stg.buf, (void *)d.stg.block_range, (void *)d.d_nodes, (void *)d.d_conn,
+                  (void *)d.d_bvh, (void *)d.d_codes, (void *)d.d_ids, (void *)d.d_left, (void *)d.d_right,
+                  (void *)d.d_parent, (void *)d.d_inner_box, (void *)d.d_nbr, (void *)d.d_coef})
+    out.push_back(p);
+}
+
+// Gives a domain's memory back, once what uses it is done.
+void free_domain(Domain &d)
+{
+  std::vector<void *> memory;
+  domain_memory(d, memory);
+  device_free(memory.data(), memory.size());
+  d = Domain();
+}
+
+}  // namespace gvr
+
 using namespace gvr;
 
 extern "C" {
@@ -376,30 +399,6 @@ int gvr_scene_create(int device, gvr_scene **out)
   return GVR_OK;
 }
 
-// The caller has waited for the device.
-static void free_domain(Domain &d)
-{
-  device_free_idle(d.d_bricks);
-  device_free_idle(d.d_cells);
-  device_free_idle(d.d_cell_rec);
-  device_free_idle(d.d_brick_range);
-  device_free_idle(d.d_brick_empty);
-  device_free_idle(d.stg.buf);
-  device_free_idle(d.stg.block_range);
-  free_hex(d);
-  d = Domain();
-}
-
-// A domain's device buffers.
-static void domain_memory(const Domain &d, std::vector<void *> &out)
-{
-  for (void *p : {(void *)d.d_bricks, (void *)d.d_cells, (void *)d.d_cell_rec, (void *)d.d_brick_range,
-                  (void *)d.d_brick_empty, d.stg.buf, (void *)d.stg.block_range, (void *)d.d_nodes, (void *)d.d_conn,
-                  (void *)d.d_bvh, (void *)d.d_codes, (void *)d.d_ids, (void *)d.d_left, (void *)d.d_right,
-                  (void *)d.d_parent, (void *)d.d_inner_box, (void *)d.d_nbr, (void *)d.d_coef})
-    out.push_back(p);
-}
-
 int gvr_scene_destroy(gvr_scene *s)
 {
   if (!s) return GVR_OK;
@@ -542,14 +541,13 @@ static int add_structured(gvr_scene *s, int kind, const int dims[3], const doubl
     e = device_alloc((void **)&d.d_cell_rec, sizeof(RectCell) * rec.size());
     if (e != cudaSuccess) return cuda_error(e, "allocate coords");
     e = cudaMemcpy(d.d_cell_rec, rec.data(), sizeof(RectCell) * rec.size(), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) { cudaDeviceSynchronize(); free_domain(d); return cuda_error(e, "copy coords"); }
+    if (e != cudaSuccess) { free_domain(d); return cuda_error(e, "copy coords"); }
     d.dev.cell_rec = d.d_cell_rec;
   }
   if (assoc == GVR_ASSOC_VERTEX) {
     d.n_values = (size_t)dims[0] * dims[1] * dims[2];
     d.n_bricks = (int64_t)d.dev.nbrick[0] * d.dev.nbrick[1] * d.dev.nbrick[2];
     if (d.n_bricks * brick_floats(d.dev.bshift) >= (int64_t)1 << 31) {
-      cudaDeviceSynchronize();
       free_domain(d);
       return set_error(GVR_ERR_UNSUPPORTED,
                        "a domain's bricked field must hold < 2^31 floats (about 1290^3 nodes); "
@@ -563,13 +561,13 @@ static int add_structured(gvr_scene *s, int kind, const int dims[3], const doubl
     d.n_values = (size_t)(dims[0] - 1) * (dims[1] - 1) * (dims[2] - 1);
     e = device_alloc((void **)&d.d_cells, sizeof(float) * d.n_values);
   }
-  if (e != cudaSuccess) { cudaDeviceSynchronize(); free_domain(d); return cuda_error(e, "allocate field"); }
+  if (e != cudaSuccess) { free_domain(d); return cuda_error(e, "allocate field"); }
   d.dev.bricks = d.d_bricks;
   d.dev.cells = d.d_cells;
   d.dev.brick_range = d.d_brick_range;
   d.dev.brick_empty = d.d_brick_empty;
   int rc = upload_field(s, d, field, dtype, stride, location);
-  if (rc != GVR_OK) { cudaDeviceSynchronize(); free_domain(d); return rc; }
+  if (rc != GVR_OK) { free_domain(d); return rc; }
   s->domains.push_back(d);
   s->table_dirty = true;
   if (domain_id) *domain_id = (int)s->domains.size() - 1;

@@ -17,6 +17,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 
 #include "gvr_hex_device.cuh"
 
@@ -559,28 +560,12 @@ cudaError_t stage(const void *src, size_t bytes, int on_device, void **owned, co
 
 }  // namespace
 
-// The caller has waited for the device.
-void free_hex(Domain &d)
+// Gives memory back once what uses it is done; the wait's refusal is rc's error
+// where there is none yet.
+static int free_after(std::initializer_list<void *> list, int rc, const char *what)
 {
-  device_free_idle(d.d_nodes);
-  device_free_idle(d.d_conn);
-  device_free_idle(d.d_bvh);
-  device_free_idle(d.d_codes);
-  device_free_idle(d.d_ids);
-  device_free_idle(d.d_left);
-  device_free_idle(d.d_right);
-  device_free_idle(d.d_parent);
-  device_free_idle(d.d_inner_box);
-  device_free_idle(d.d_nbr);
-  d.d_nbr = nullptr;
-  device_free_idle(d.d_coef);
-  d.d_coef = nullptr;
-  d.d_nodes = nullptr;
-  d.d_conn = nullptr;
-  d.d_bvh = nullptr;
-  d.d_codes = d.d_ids = nullptr;
-  d.d_left = d.d_right = d.d_parent = nullptr;
-  d.d_inner_box = nullptr;
+  const cudaError_t e = device_free(list.begin(), list.size());
+  return rc == GVR_OK && e != cudaSuccess ? cuda_error(e, what) : rc;
 }
 
 // Range of the vertex field held in nodes[].w.
@@ -688,11 +673,7 @@ static int sort_neighbours(Domain &d)
   count_launch();
   NB_TRY(cudaGetLastError(), "neighbour launch");
 done:
-  cudaDeviceSynchronize();
-  for (void *p : {(void *)key, (void *)key_tmp, (void *)key2, (void *)key2_tmp, (void *)face, (void *)face_tmp,
-                  (void *)scr})
-    device_free_idle(p);
-  return rc;
+  return free_after({key, key_tmp, key2, key2_tmp, face, face_tmp, scr}, rc, "neighbours");
 }
 
 // Face-neighbour table: 6 cell ids per cell (-1 on the boundary).
@@ -723,8 +704,7 @@ static int build_neighbours(Domain &d)
   NB_TRY(cudaMemcpy(&crowded, d_crowded, sizeof(int), cudaMemcpyDeviceToHost), "neighbours");
 done:
 #undef NB_TRY
-  cudaDeviceSynchronize();
-  for (void *p : {(void *)off, (void *)slot, (void *)bucket, (void *)scan_tmp, (void *)d_crowded}) device_free_idle(p);
+  rc = free_after({off, slot, bucket, scan_tmp, d_crowded}, rc, "neighbours");
   if (rc == GVR_OK && crowded) rc = sort_neighbours(d);
   d.nbr_build_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
   return rc;
@@ -846,17 +826,8 @@ static int build_hex(Domain &d, const void *x, const void *y, const void *z, int
   }
 done:
 #undef HEX_TRY
-  if (rc != GVR_OK) cudaDeviceSynchronize();   // otherwise the tree was waited for
-  for (void *p : own) device_free_idle(p);
-  device_free_idle(d_flag);
-  device_free_idle(leaf_lo);
-  device_free_idle(leaf_hi);
-  device_free_idle(part);
-  device_free_idle(keys_tmp);
-  device_free_idle(vals_tmp);
-  device_free_idle(sort_scr);
-  device_free_idle(counters);
-  device_free_idle(range);
+  rc = free_after({own[0], own[1], own[2], own[3], own[4], d_flag, leaf_lo, leaf_hi, part, keys_tmp, vals_tmp, sort_scr,
+                   counters, range}, rc, "BVH build");
   d.bvh_build_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
   if (rc == GVR_OK) rc = build_neighbours(d);
   d.dev.hex_nbr = d.d_nbr;
@@ -907,11 +878,7 @@ int gvr_scene_add_hex(gvr_scene *s, int64_t n_nodes, const void *x, const void *
   int rc = build_hex(d, x, y, z, coord_dtype, conn, conn_int64 ? 1 : 0, field, dtype, association,
                      location);
   if (rc != GVR_OK) {
-    cudaDeviceSynchronize();
-    free_hex(d);
-    device_free(d.d_cells);
-    device_free(d.stg.buf);
-    device_free(d.stg.block_range);
+    free_domain(d);
     return rc;
   }
   s->domains.push_back(d);

@@ -271,12 +271,12 @@ cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
 // library: usable at once on any stream. device_free waits for the device
 // first, as cudaFree does. Where the wait is refused (a capture in progress)
 // the memory may still be in use: it is kept, and freed after a later call's
-// wait; the refusal is returned. device_free_idle is for a caller that has
-// waited.
+// wait; the refusal is returned.
 cudaError_t device_alloc(void **ptr, size_t bytes);
 cudaError_t device_free(void *const *ptrs, size_t n);
 inline cudaError_t device_free(void *ptr) { return device_free(&ptr, 1); }
-void device_free_idle(void *ptr);
+// a domain's memory, and the domain empty
+void free_domain(Domain &d);
 
 // kernels launched by this library since it was loaded
 void count_launch(int n = 1);
@@ -330,7 +330,6 @@ cudaError_t radix_sort_pairs(K *keys, uint32_t *vals, K *keys_tmp, uint32_t *val
                              int64_t n, int key_bits, uint32_t *scratch, cudaStream_t stream);
 
 // hexahedral domains (gvr_hex.cu)
-void free_hex(Domain &d);
 int hex_update_field(Domain &d, const void *field, int dtype, int64_t stride, int location);
 
 // march kernel (gvr_march.cu); CTA i renders tile d_order[i] (a linear

@@ -145,22 +145,6 @@ cudaError_t device_alloc(void **ptr, size_t bytes)
   return e;
 }
 
-void device_free_idle(void *ptr)
-{
-  if (!ptr) return;
-  int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxPoolDevices) {
-    cudaFree(ptr);
-    return;
-  }
-  cudaStream_t stream;
-  {
-    std::lock_guard<std::mutex> lock(g_pool_mu);
-    stream = g_scene_streams[device];
-  }
-  cudaFreeAsync(ptr, stream);
-}
-
 // The device's default memory pool gives its free memory back to the
 // system at every synchronisation (release threshold 0), so a call that
 // allocates tens of MB of scratch and synchronises would map fresh pages

@@ -95,3 +95,49 @@ def test_destroy_beside_refusing_capture():
     assert np.array_equal(b.render(cam, p)[0], image)
     b.close()
     assert free_bytes() == before
+
+
+def crowded_mesh(n=3000):
+    """n hexahedra around one node: too many for a bucket, so the faces are sorted."""
+    a = np.linspace(0.0, 2.0 * np.pi, n + 1)[:-1]
+    ring = lambda r, z: np.stack([r * np.cos(a), r * np.sin(a), np.full(n, z)], 1)
+    pts = np.concatenate([[[0, 0, 0], [0, 0, 1]], ring(0.5, 0.0), ring(0.5, 1.0), ring(1.0, 0.0), ring(1.0, 1.0)])
+    i = np.arange(n)
+    j = (i + 1) % n
+    node = lambda k, q: 2 + k * n + q
+    conn = np.stack([np.zeros(n, int), node(0, i), node(2, i), node(0, j),
+                     np.ones(n, int), node(1, i), node(3, i), node(1, j)], 1)
+    return pts, conn
+
+
+def hex_scene(pts, conn):
+    sc = S.Scene(0)
+    sc.add_hex(*[np.ascontiguousarray(pts[:, k]) for k in range(3)], conn, pts[:, 2] + pts[:, 0])
+    return sc
+
+
+def test_failed_adds_give_their_memory_back():
+    """Refused fields and meshes leave nothing behind, and the scene as it was."""
+    pts, conn = crowded_mesh()
+    hex_scene(pts, conn).close()
+    wl, cam, p, before = two_domains()
+    sc = make(wl)
+    image = sc.render(cam, p)[0]
+    n = 160
+    bad = np.zeros((n, n, n), np.float32)
+    bad[-1, -1, -1] = np.nan
+    missing = conn.copy()
+    missing[-1, -1] = len(pts)
+    for _ in range(3):
+        for assoc in (N.ASSOC_VERTEX, N.ASSOC_ELEMENT):
+            with pytest.raises(N.GvrError):
+                sc.add_uniform(bad, (0, 0, 0), (1, 1, 1), association=assoc)
+            with pytest.raises(N.GvrError):
+                grid = [np.linspace(0.0, 1.0, n + (assoc == N.ASSOC_ELEMENT))] * 3
+                sc.add_rectilinear(bad, *grid, association=assoc)
+        with pytest.raises(N.GvrError):
+            sc.add_hex(*[np.ascontiguousarray(pts[:, k]) for k in range(3)], missing, pts[:, 2])
+        hex_scene(pts, conn).close()
+    assert np.array_equal(sc.render(cam, p)[0], image)
+    sc.close()
+    assert free_bytes() == before
