@@ -86,11 +86,12 @@ cudaError_t device_free(void *const *ptrs, size_t n)
   e = wait_for_device();
   if (e == cudaSuccess) {
     for (void *p : list) cudaFreeAsync(p, stream);
+    e = cudaStreamSynchronize(stream);   // until which the memory counts as used where the pool is trimmed
   } else {
-    cudaGetLastError();   // not the next launch's
     std::lock_guard<std::mutex> lock(g_pool_mu);
     g_kept[device].insert(g_kept[device].end(), list.begin(), list.end());
   }
+  if (e != cudaSuccess) cudaGetLastError();   // not the next launch's
   return e;
 }
 
@@ -98,9 +99,9 @@ cudaError_t device_free(void *const *ptrs, size_t n)
 // that cudaMalloc maps and cudaFree unmaps, each call a synchronisation: 3.9
 // of the 6.7 ms of a step with 1M new hexahedra, 1.2 of 3.4 ms of one with
 // four structured host domains. From a pool they cost a microsecond each; the
-// pool gives back what it holds beyond kScenePoolKeep at the next
-// synchronisation, all of it to gvr_scratch_trim, and when an allocation does
-// not fit. Allocations and frees are made on one stream of the pool's own on
+// pool gives back what it holds beyond kScenePoolKeep when a scene's memory is
+// freed, all of it to gvr_scratch_trim, and when an allocation of either pool
+// does not fit. Allocations and frees are made on one stream of the pool's own on
 // which nothing runs, and an allocation is waited for, so that the memory may
 // be used on any stream and from any thread.
 cudaError_t device_alloc(void **ptr, size_t bytes)
@@ -150,7 +151,10 @@ cudaError_t device_alloc(void **ptr, size_t bytes)
 // allocates tens of MB of scratch and synchronises would map fresh pages
 // every time. This library's own pool keeps what it has allocated (up to
 // its high-water mark, held until the process exits) and leaves the
-// default pool, which other libraries in the process may use, as it is.
+// default pool, which other libraries in the process may use, as it is. An
+// allocation that does not fit is tried again without what both pools hold
+// free, as much as the scenes' pool keeps; not under capture, where the trim's
+// waits are refused.
 cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream)
 {
   int device = 0;
@@ -163,6 +167,13 @@ cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream)
     if (!g_pools[device] && (e = make_pool(device, UINT64_MAX, &g_pools[device])) != cudaSuccess) return e;
     pool = g_pools[device];
   }
+  e = cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+  if (e != cudaErrorMemoryAllocation || cudaStreamIsCapturing(stream, &capture) != cudaSuccess ||
+      capture != cudaStreamCaptureStatusNone)
+    return e;
+  cudaGetLastError();
+  gvr_scratch_trim(device, 0, nullptr);
   return cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
 }
 

@@ -21,6 +21,7 @@ struct Block {
 size_t capacity = 1 << 20;     // of the device
 bool capturing = false;        // a capture that refuses unsafe calls
 bool device_sync_seen = false;
+int trims = 0;
 cudaError_t last = cudaSuccess;
 std::set<Pool *> pools;
 std::map<void *, Block> blocks;
@@ -96,6 +97,7 @@ cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t p, cudaMemPoolAttr, void *v)
 }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t p, size_t n)
 {
+  ++trims;
   Pool *q = (Pool *)p;
   const size_t keep = n > q->used ? n - q->used : 0;
   if (q->free > keep) q->free = keep;
@@ -170,9 +172,39 @@ static void refused_allocation()
   last = cudaSuccess;
 }
 
+// What either pool holds free is given back where the other's allocation does
+// not fit, not under capture; and the device's memory is what it was.
+static void out_of_memory()
+{
+  void *a, *s;
+  trims = 0;
+  CHECK(device_alloc(&a, 800000) == cudaSuccess && device_free(a) == cudaSuccess);
+  CHECK(scratch_alloc(&s, 900000, nullptr) == cudaSuccess);   // the scenes' pool made room
+  CHECK(trims > 0 && last == cudaSuccess);
+  CHECK(scratch_alloc(&a, 900000, nullptr) == cudaErrorMemoryAllocation && blocks.count(s));
+  last = cudaSuccess;
+  CHECK(cudaFreeAsync(s, nullptr) == cudaSuccess);
+  trims = 0;
+  CHECK(device_alloc(&a, 700000) == cudaSuccess);             // the scratch pool did
+  CHECK(trims > 0 && last == cudaSuccess);
+  CHECK(device_alloc(&s, 700000) == cudaErrorMemoryAllocation && s == nullptr);
+  last = cudaSuccess;
+  CHECK(device_free(a) == cudaSuccess);
+  capturing = true;
+  trims = 0;
+  CHECK(scratch_alloc(&s, 900000, nullptr) == cudaErrorMemoryAllocation && trims == 0);
+  capturing = false;
+  last = cudaSuccess;
+  CHECK(gvr_scratch_trim(0, 0, nullptr) == GVR_OK);
+  size_t held = 0;
+  for (Pool *p : pools) held += p->used + p->free;
+  CHECK(held == 0);
+}
+
 int main()
 {
   for (int then = 0; then < 3; ++then) refused_wait(then);
   refused_allocation();
+  out_of_memory();
   return checks_failed != 0;
 }

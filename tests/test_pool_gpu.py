@@ -1,5 +1,6 @@
-"""Scenes' memory on the device: destroying a scene beside another thread's
-stream capture.
+"""Scenes' memory on the device: scenes destroyed beside another thread's stream
+capture, adds that fail, what the pool keeps and gives back, scenes of two
+threads.
 """
 import ctypes as C
 import threading
@@ -67,6 +68,7 @@ def two_domains():
     sc.render(cam, p)
     sc.close()
     assert Capture(THREAD_LOCAL).end()
+    torch.zeros(1, device="cuda")
     return wl, cam, p, free_bytes()
 
 
@@ -141,3 +143,59 @@ def test_failed_adds_give_their_memory_back():
     assert np.array_equal(sc.render(cam, p)[0], image)
     sc.close()
     assert free_bytes() == before
+
+
+def available():
+    return torch.cuda.mem_get_info(0)[0]
+
+
+def test_pool_is_bounded_and_given_back():
+    """Scenes that come and go take the same memory again; at most 4 GiB stay
+    reserved when one is gone, and a trim gives that back too, with no wait in
+    between."""
+    wl, cam, p, before = two_domains()
+    scenes = []
+    for _ in range(6):
+        sc = make(wl)
+        sc.render(cam, p)
+        sc.close()
+        scenes.append(before - available())
+    assert scenes[0] > 0 and max(scenes) == scenes[0], scenes
+    cells = torch.zeros((1300, 1100, 1100), device="cuda")      # 6.3 GB
+    held = available()
+    with S.Scene(0) as sc:
+        sc.add_uniform(cells, (0, 0, 0), (1, 1, 1), association=N.ASSOC_ELEMENT)
+        assert held - available() > 5 << 30
+    assert held + scenes[0] - available() <= (4 << 30) + (64 << 20)
+    N.scratch_trim(0, 0)
+    assert available() == held + scenes[0]
+    del cells
+    torch.cuda.empty_cache()
+
+
+def test_scenes_of_two_threads():
+    """Threads that make, render and destroy scenes get their own images."""
+    wls = [W.plain_small(n=n, width=96, height=80, parts=(2, 1, 1)) for n in (40, 72)]
+
+    def images(wl, turns):
+        cam, p = V.workload_camera(wl), V.workload_params(wl)
+        out = []
+        for _ in range(turns):
+            sc = make(wl)
+            out.append(sc.render(cam, p)[0])
+            sc.close()
+        return out
+
+    want = [images(wl, 1)[0] for wl in wls]
+    got = [None, None]
+
+    def work(k):
+        got[k] = images(wls[k], 25)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(2):
+        assert all(np.array_equal(g, want[k]) for g in got[k])
