@@ -387,9 +387,10 @@ __global__ void pixel_emit_kernel(const Partial *__restrict__ in, const uint32_t
 // Slots: the dense path while the pixels are no more than twice the records.
 // Every pixel has kSlots places for record indices (place s of all pixels
 // together: neighbouring records mostly take the same place of neighbouring
-// pixels), which a record's atomic on the pixel's count hands out directly, so there is no bucket offset to scan
-// for and no second pass over the records before they are blended; records
-// beyond the places hang on the pixel in a list. Bound by memory: the records
+// pixels), which a record's atomic on the pixel's count hands out directly, so
+// there is no bucket offset to scan for and no second pass over the records
+// before they are blended; records beyond the places hang on the pixel in a
+// list. Bound by memory: the records
 // are read twice, once for their pixel ids (24-byte records, so every sector of
 // them) and once to blend, the index places stay in L2. 8 images of 1024^2 at
 // 80% cover (6.7M records, 161 MB): the histogram, three scans, bucket and emit
@@ -398,7 +399,8 @@ __global__ void pixel_emit_kernel(const Partial *__restrict__ in, const uint32_t
 // at 3 CTAs per SM, 92 at 5, where it spills).
 // ---------------------------------------------------------------------------
 constexpr int kSlots = 8;
-constexpr int kSlotTile = 1024;   // pixels per CTA of the last two passes
+constexpr int kSlotThreads = 256;
+constexpr uint32_t kWarpDeep = 1024;   // records of a pixel that a warp orders alone
 
 // Word-sized loads of a record, or 8-byte ones where the array is aligned.
 template <bool WIDE>
@@ -440,9 +442,11 @@ slot_kernel(const Partial *__restrict__ in, int64_t n, int lo, int64_t r, uint32
   }
 }
 
-// Pixels with one record and with more, per tile; the CTA that finishes last
-// turns the tiles' numbers into exclusive prefixes and writes the totals.
-__global__ void __launch_bounds__(256)
+// Pixels with one record and with more, per tile of ROWS x 256; the CTA that
+// finishes last turns the tiles' numbers into exclusive prefixes and writes the
+// totals.
+template <int ROWS>
+__global__ void __launch_bounds__(kSlotThreads)
 slot_sums_kernel(const uint32_t *__restrict__ cnt, int64_t r, uint2 *__restrict__ sums, int tiles,
                  unsigned *__restrict__ finished, uint32_t *__restrict__ totals)
 {
@@ -450,9 +454,11 @@ slot_sums_kernel(const uint32_t *__restrict__ cnt, int64_t r, uint2 *__restrict_
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned one = 0, more = 0;
-  const int64_t p0 = (int64_t)blockIdx.x * kSlotTile;
-  for (int k = threadIdx.x; k < kSlotTile; k += 256) {
-    const uint32_t c = p0 + k < r ? cnt[p0 + k] : 0u;
+  const int64_t p0 = (int64_t)blockIdx.x * (ROWS * kSlotThreads);
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) {
+    const int64_t p = p0 + q * kSlotThreads + threadIdx.x;
+    const uint32_t c = p < r ? cnt[p] : 0u;
     one += c == 1;
     more += c > 1;
   }
@@ -505,27 +511,78 @@ slot_sums_kernel(const uint32_t *__restrict__ cnt, int64_t r, uint2 *__restrict_
   }
 }
 
+// Blends a pixel's c records, whose indices are rows[0 .. c - 1].y, in (depth,
+// input index) order: by one warp, or by all of a CTA (the last blend by its
+// first warp alone). Each record's place is the number of those before it;
+// next[] of the pixel's own records, which nothing walks any more, holds the
+// order. Every lane of the blending warp gets the result.
+template <bool CTA, bool WIDE>
+__device__ __forceinline__ Partial blend_deep(const Partial *__restrict__ in, uint2 *rows, uint32_t c, uint32_t *next)
+{
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t t = CTA ? threadIdx.x : lane, step = CTA ? kSlotThreads : 32;
+  const auto meet = [] {
+    if (CTA) __syncthreads();
+    else __syncwarp();
+  };
+  for (uint32_t j = t; j < c; j += step) rows[j].x = order_bits(__ldg(&in[rows[j].y].depth));
+  meet();
+  for (uint32_t j = t; j < c; j += step) {
+    const uint2 mine = rows[j];
+    uint32_t rank = 0;
+    for (uint32_t q = 0; q < c; ++q) {
+      const uint2 o = rows[q];
+      rank += before(o.x, o.y, mine.x, mine.y);
+    }
+    next[rows[rank].y] = mine.y;
+  }
+  meet();
+  Partial res{};
+  if (CTA && threadIdx.x >= 32) return res;
+  for (uint32_t j0 = 0; j0 < c; j0 += 32) {
+    Partial mine{};
+    if (j0 + lane < c) mine = load_partial<WIDE>(in + next[rows[j0 + lane].y]);
+    const uint32_t m = min(32u, c - j0);
+    for (uint32_t k = 0; k < m; ++k) {
+      Partial rec;
+      rec.pixel_id = __shfl_sync(0xffffffffu, mine.pixel_id, k);
+      rec.depth = __shfl_sync(0xffffffffu, mine.depth, k);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) rec.rgb[a] = __shfl_sync(0xffffffffu, mine.rgb[a], k);
+      rec.alpha = __shfl_sync(0xffffffffu, mine.alpha, k);
+      if (j0 + k == 0) res = rec;
+      else blend_into(res, rec);
+    }
+  }
+  return res;
+}
+
 // One thread per pixel: copy its record or blend its records in (depth, input
 // index) order. Up to kSlots records are loaded whole, so that each is read
 // once, and ordered by Batcher's odd-even merge network (19 exchanges) with
-// their colours; more are taken one by one, each the next in order among the
-// pixel's places and list. n_out (may be NULL) receives the count, -1 when a
-// record was outside the caller's range.
-template <bool WIDE>
-__global__ void __launch_bounds__(256, 4)
+// their colours. Up to kLocalSort are ordered by insertion in local arrays,
+// their indices, then their depths, then the records loaded several at a time.
+// Of more, the thread writes the indices down and a warp blends them later, all
+// of the CTA's warps together those of more than kWarpDeep: 64 images of 256^2,
+// 480 us (sorted by insertion, a thread a pixel, 1110 us; by the whole CTA one
+// after the other, with one thread walking the list, 11 ms); one pixel of 5000
+// records 2.9 ms (861 by insertion). n_out (may be NULL)
+// receives the count, -1 when a record was outside the caller's range.
+template <int ROWS, bool WIDE>
+__global__ void __launch_bounds__(kSlotThreads, 4)
 slot_emit_kernel(const Partial *__restrict__ in, const uint32_t *__restrict__ cnt,
-                 const uint32_t *__restrict__ place, const uint32_t *__restrict__ head,
-                 const uint32_t *__restrict__ next, const uint2 *__restrict__ sums, int64_t r,
-                 Partial *__restrict__ out, const uint32_t *__restrict__ totals, const unsigned *__restrict__ bad,
-                 int64_t *__restrict__ n_out, uint32_t *rows, int64_t n, uint32_t *__restrict__ used)
+                 const uint32_t *__restrict__ place, const uint32_t *__restrict__ head, uint32_t *next,
+                 const uint2 *__restrict__ sums, int64_t r, Partial *__restrict__ out,
+                 const uint32_t *__restrict__ totals, const unsigned *__restrict__ bad,
+                 int64_t *__restrict__ n_out, uint2 *rows, uint32_t *__restrict__ used)
 {
-  constexpr int kRows = kSlotTile / 256;    // pixels per thread
-  __shared__ uint2 part[kRows][8];
-  __shared__ int n_deep;                    // pixels deeper than kLocalSort: place in the tile, output
-  __shared__ int deep[kSlotTile];
-  __shared__ uint32_t deep_out[kSlotTile];
-  __shared__ uint32_t row;
-  if (threadIdx.x == 0) n_deep = 0;
+  constexpr int kTile = ROWS * kSlotThreads;   // pixels per CTA
+  __shared__ uint2 part[ROWS][8];
+  __shared__ int n_deep, n_deepest;       // pixels deeper than kLocalSort, and than kWarpDeep
+  // of each: place in the tile, output, rows; the deepest from the end
+  __shared__ int deep[kTile];
+  __shared__ uint32_t deep_out[kTile], deep_row[kTile];
+  if (threadIdx.x == 0) n_deep = n_deepest = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t n_unique = totals[0];
@@ -533,10 +590,10 @@ slot_emit_kernel(const Partial *__restrict__ in, const uint32_t *__restrict__ cn
     *n_out = *bad ? -1 : (int64_t)n_unique + totals[1];
   // the counts and output slots of all of a thread's pixels first, so that
   // nothing is waited for between them
-  __shared__ uint32_t counts[kRows][256];
+  __shared__ uint32_t counts[ROWS][kSlotThreads];
 #pragma unroll
-  for (int q = 0; q < kRows; ++q) {
-    const int64_t p = (int64_t)blockIdx.x * kSlotTile + q * 256 + threadIdx.x;
+  for (int q = 0; q < ROWS; ++q) {
+    const int64_t p = (int64_t)blockIdx.x * kTile + q * kSlotThreads + threadIdx.x;
     const uint32_t c = p < r ? __ldg(cnt + p) : 0u;
     const unsigned ones = __ballot_sync(0xffffffffu, c == 1), mores = __ballot_sync(0xffffffffu, c > 1);
     counts[q][threadIdx.x] = c;
@@ -545,8 +602,8 @@ slot_emit_kernel(const Partial *__restrict__ in, const uint32_t *__restrict__ cn
   __syncthreads();
   uint2 base = sums[blockIdx.x];
 #pragma unroll 1
-  for (int q = 0; q < kRows; ++q) {
-    const int64_t p = (int64_t)blockIdx.x * kSlotTile + q * 256 + threadIdx.x;
+  for (int q = 0; q < ROWS; ++q) {
+    const int64_t p = (int64_t)blockIdx.x * kTile + q * kSlotThreads + threadIdx.x;
     const uint32_t c = counts[q][threadIdx.x];
     uint32_t upos = base.x + __popc(__ballot_sync(0xffffffffu, c == 1) & ((1u << lane) - 1u));
     uint32_t mpos = base.y + __popc(__ballot_sync(0xffffffffu, c > 1) & ((1u << lane) - 1u));
@@ -615,56 +672,47 @@ slot_emit_kernel(const Partial *__restrict__ in, const uint32_t *__restrict__ cn
         if ((uint32_t)j < c) blend_into(res, rec[j]);
     } else if (c <= kLocalSort) {
       uint32_t key[kLocalSort], idx[kLocalSort];
-      uint32_t held = 0;
-      auto insert = [&](uint32_t i) {
-        const uint32_t k = order_bits(__ldg(&in[i].depth));
-        uint32_t q = held++;
-        while (q > 0 && before(k, i, key[q - 1], idx[q - 1])) {
-          key[q] = key[q - 1];
-          idx[q] = idx[q - 1];
-          --q;
+      uint32_t held = kSlots;
+#pragma unroll
+      for (int m = 0; m < kSlots; ++m) idx[m] = __ldg(seg + m * r);
+      for (uint32_t t = head[p]; t; t = next[t - 1]) idx[held++] = t - 1;
+#pragma unroll 8
+      for (uint32_t j = 0; j < c; ++j) key[j] = order_bits(__ldg(&in[idx[j]].depth));
+      for (uint32_t j = 1; j < c; ++j) {
+        const uint32_t k = key[j], i = idx[j];
+        uint32_t to = j;
+        while (to > 0 && before(k, i, key[to - 1], idx[to - 1])) {
+          key[to] = key[to - 1];
+          idx[to] = idx[to - 1];
+          --to;
         }
-        key[q] = k;
-        idx[q] = i;
-      };
-      for (int m = 0; m < kSlots; ++m) insert(seg[m * r]);
-      for (uint32_t t = head[p]; t; t = next[t - 1]) insert(t - 1);
+        key[to] = k;
+        idx[to] = i;
+      }
       res = load_partial<WIDE>(in + idx[0]);
+#pragma unroll 4
       for (uint32_t j = 1; j < c; ++j) blend_into(res, load_partial<WIDE>(in + idx[j]));
     } else {
-      const int d = atomicAdd(&n_deep, 1);
-      deep[d] = q * 256 + (int)threadIdx.x;
+      const uint32_t row = atomicAdd(used, c);
+      uint32_t m = row;
+      for (int j = 0; j < kSlots; ++j) rows[m++].y = seg[j * r];
+      for (uint32_t t = head[p]; t; t = next[t - 1]) rows[m++].y = t - 1;
+      const int d = c <= kWarpDeep ? atomicAdd(&n_deep, 1) : kTile - 1 - atomicAdd(&n_deepest, 1);
+      deep[d] = q * kSlotThreads + (int)threadIdx.x;
       deep_out[d] = n_unique + mpos;
+      deep_row[d] = row;
       continue;
     }
     out[n_unique + mpos] = res;
   }
   __syncthreads();
-  for (int d = 0; d < n_deep; ++d) {
-    const int64_t p = (int64_t)blockIdx.x * kSlotTile + deep[d];
-    const uint32_t c = cnt[p];
-    if (threadIdx.x == 0) {
-      row = atomicAdd(used, c);
-      uint32_t m = row;
-      for (int j = 0; j < kSlots; ++j) rows[m++] = place[j * r + p];
-      for (uint32_t t = head[p]; t; t = next[t - 1]) rows[m++] = t - 1;
-    }
-    __syncthreads();
-    const uint32_t *from = rows + row;
-    uint32_t *sorted = rows + n + row;
-    for (uint32_t j = threadIdx.x; j < c; j += 256) {
-      const uint32_t i = from[j], k = order_bits(__ldg(&in[i].depth));
-      uint32_t rank = 0;
-      for (uint32_t q = 0; q < c; ++q) rank += before(order_bits(__ldg(&in[from[q]].depth)), from[q], k, i);
-      sorted[rank] = i;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      Partial res = load_partial<WIDE>(in + sorted[0]);
-      for (uint32_t j = 1; j < c; ++j) blend_into(res, load_partial<WIDE>(in + sorted[j]));
-      out[deep_out[d]] = res;
-    }
-    __syncthreads();
+  for (int d = warp; d < n_deep; d += kSlotThreads / 32) {
+    const Partial res = blend_deep<false, WIDE>(in, rows + deep_row[d], cnt[(int64_t)blockIdx.x * kTile + deep[d]], next);
+    if (lane == 0) out[deep_out[d]] = res;
+  }
+  for (int d = kTile - 1; d > kTile - 1 - n_deepest; --d) {
+    const Partial res = blend_deep<true, WIDE>(in, rows + deep_row[d], cnt[(int64_t)blockIdx.x * kTile + deep[d]], next);
+    if (threadIdx.x == 0) out[deep_out[d]] = res;
   }
 }
 
@@ -701,12 +749,32 @@ size_t sorted_bytes(int64_t n)
 
 // Whether the slots serve: their places are read for every pixel, and take 32
 // bytes of scratch each.
-bool use_slots(int64_t n, int64_t r) { return r <= 2 * n && (r + kSlotTile - 1) / kSlotTile < ((int64_t)1 << 30); }
+bool use_slots(int64_t n, int64_t r) { return r <= 2 * n; }
 
 size_t slot_bytes(int64_t n, int64_t r)
 {
-  return 256 * 9 + ((2 + kSlots) * (size_t)r + 3 * (size_t)n + 2 * (size_t)((r + kSlotTile - 1) / kSlotTile) + 8) *
+  return 256 * 9 + ((2 + kSlots) * (size_t)r + 3 * (size_t)n + 2 * (size_t)((r + kSlotThreads - 1) / kSlotThreads) + 8) *
                        sizeof(uint32_t);
+}
+
+// Four pixels per thread of the last two passes, whose loads overlap, where the
+// records fit their places on average and the CTAs of 1024 pixels fill the SMs
+// once, four each; otherwise one, as the few CTAs or a thread's deep pixels one
+// after the other make the pass longer. 8 images of 1024^2 at 80%: 116 us with
+// four, 135 with one; 12 images (9.6 records a pixel) 347 and 324; 8 of 256^2:
+// 41 and 36.
+constexpr int64_t kSlotWave = 152 * 4;
+bool four_per_thread(int64_t n, int64_t r) { return n <= kSlots * r && r >= kSlotWave * 4 * kSlotThreads; }
+
+template <int ROWS>
+void launch_slot_passes(const Partial *in, int64_t r, Partial *out, const uint32_t *cnt, const uint32_t *place,
+                        const uint32_t *head, uint32_t *next, uint2 *sums, uint32_t *totals, unsigned *bad,
+                        unsigned *finished, uint32_t *used, int64_t *n_out, uint2 *rows, cudaStream_t st)
+{
+  const unsigned tiles = (unsigned)((r + ROWS * kSlotThreads - 1) / (ROWS * kSlotThreads));
+  slot_sums_kernel<ROWS><<<tiles, kSlotThreads, 0, st>>>(cnt, r, sums, (int)tiles, finished, totals);
+  const auto emit = ((uintptr_t)in & 7) == 0 ? slot_emit_kernel<ROWS, true> : slot_emit_kernel<ROWS, false>;
+  emit<<<tiles, kSlotThreads, 0, st>>>(in, cnt, place, head, next, sums, r, out, totals, bad, n_out, rows, used);
 }
 
 // Dense pixel ids, no more than twice as many as records: slots, tile sums,
@@ -714,24 +782,18 @@ size_t slot_bytes(int64_t n, int64_t r)
 cudaError_t composite_slots(const Partial *in, int64_t n, int lo, int64_t r, Partial *out, Arena &a,
                             uint32_t *totals, int64_t *n_out, cudaStream_t st)
 {
-  const int tiles = (int)((r + kSlotTile - 1) / kSlotTile);
   uint32_t *place = a.take<uint32_t>(kSlots * (size_t)r);
   uint32_t *next = a.take<uint32_t>(n);
-  uint32_t *rows = a.take<uint32_t>(2 * (size_t)n);   // deep pixels' records, then in order
-  uint2 *sums = a.take<uint2>(tiles);
+  uint2 *rows = a.take<uint2>(n);   // deep pixels' records: key, index
+  uint2 *sums = a.take<uint2>((r + kSlotThreads - 1) / kSlotThreads);
   // counts, list heads and the three words are cleared together
   uint32_t *cnt = a.take<uint32_t>(2 * (size_t)r + 3), *head = cnt + r;
   unsigned *bad = head + r, *finished = bad + 1, *used = bad + 2;
   cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (2 * (size_t)r + 3), st);
   if (e != cudaSuccess) return e;
   slot_kernel<<<grid_of(n), 256, 0, st>>>(in, n, lo, r, cnt, place, head, next, bad);
-  slot_sums_kernel<<<(unsigned)tiles, 256, 0, st>>>(cnt, r, sums, tiles, finished, totals);
-  if (((uintptr_t)in & 7) == 0)
-    slot_emit_kernel<true><<<(unsigned)tiles, 256, 0, st>>>(in, cnt, place, head, next, sums, r, out, totals, bad, n_out,
-                                                               rows, n, used);
-  else
-    slot_emit_kernel<false><<<(unsigned)tiles, 256, 0, st>>>(in, cnt, place, head, next, sums, r, out, totals, bad, n_out,
-                                                               rows, n, used);
+  const auto passes = four_per_thread(n, r) ? launch_slot_passes<4> : launch_slot_passes<1>;
+  passes(in, r, out, cnt, place, head, next, sums, totals, bad, finished, used, n_out, rows, st);
   count_launch(3);
   return cudaGetLastError();
 }
