@@ -510,8 +510,8 @@ static int add_structured(gvr_scene *s, int kind, const int dims[3], const doubl
     for (int a = 0; a < 3; ++a) {
       if (!coords[a]) return set_error(GVR_ERR_INVALID_ARGUMENT, "rectilinear coordinates are NULL");
       const int n = dims[a] - 1;
-      const size_t first = rec.size();
-      rec.resize(first + 2 * (size_t)n);
+      const size_t first = rec.size(), list = (size_t)rect_list(dims[a]);
+      rec.resize(first + 2 * list, RectCell{0.f, 1.f, 1.f, INFINITY, 0});
       float x0 = (float)coords[a][0];
       d.dev.lo[a] = x0;
       for (int i = 0; i < n; ++i) {
@@ -525,8 +525,9 @@ static int add_structured(gvr_scene *s, int kind, const int dims[3], const doubl
         f.ahead = i + 1 < n ? x1 : INFINITY;
         f.share = assoc == GVR_ASSOC_ELEMENT
                       ? i : (int)((i >> sh) * of_brick + (i & (brick_cells(sh) - 1)) * in_brick);
-        rec[first + n + i] = f;
-        rec[first + n + i].ahead = i > 0 ? -x0 : INFINITY;
+        RectCell &b = rec[first + list + n - 1 - i];
+        b = f;
+        b.ahead = i > 0 ? -x0 : INFINITY;
         x0 = x1;
       }
       in_brick *= brick_nodes(sh);
@@ -1001,6 +1002,23 @@ static int march_mode(const gvr_scene *s)
   return mode;
 }
 
+// Whether a step is two cells and more in every rectilinear domain, along its
+// diagonal on average.
+static bool long_steps(const gvr_scene *s, float sample_dist)
+{
+  for (const Domain &d : s->domains) {
+    if (d.dev.kind != GVR_DOMAIN_RECTILINEAR) continue;
+    double cells = 0, length = 0;
+    for (int a = 0; a < 3; ++a) {
+      const double n = d.dev.dims[a] - 1, w = d.bounds[2 * a + 1] - d.bounds[2 * a];
+      cells += n * n;
+      length += w * w;
+    }
+    if (!(sample_dist * std::sqrt(cells / length) >= 2)) return false;
+  }
+  return true;
+}
+
 static int render_one(gvr_scene *s, const gvr_camera *camera, const gvr_render_params *p,
                       float *rgba, float *depth, int out_location, void *stream,
                       uint64_t *samples_out, bool over);
@@ -1234,9 +1252,10 @@ static int render_one(gvr_scene *s, const gvr_camera *camera, const gvr_render_p
                       samples_out ? s->d_counters : nullptr, s->tuning, d_order, order,
                       s->d_counters + 1, st);
   } else {
+    const int mode = std::max<int>(march_mode(s), over ? kMarchCells : kMarchUniform);
     e = launch_march(s->d_domains, view, mp, s->d_lut, d_rgba, d_depth,
-                     samples_out ? s->d_counters : nullptr, s->tuning, std::max<int>(march_mode(s), over ? kMarchCells : kMarchUniform),
-                     d_order, st);
+                     samples_out ? s->d_counters : nullptr, s->tuning, mode,
+                     mode == kMarchRect && long_steps(s, p->sample_dist), d_order, st);
   }
   if (e != cudaSuccess) return cuda_error(e, "march kernel launch");
   if (out_location == GVR_MEM_HOST) {

@@ -46,12 +46,17 @@ constexpr int kMarchTile = 16;      // march kernel: one CTA per 16x16-pixel til
 // A cell of a rectilinear domain's axis, for rays in one of its directions:
 // first node, width and 1 / width; the node ahead times the direction's sign
 // (infinite in the last cell); the cell's share of a vertex field's brick
-// offset, or its own index for a cell-centred field. An axis of n cells has n
-// records for rays along it, then n for rays against it.
+// offset, or its own index for a cell-centred field. An axis of n cells has a
+// list of n records for rays along it and then one, from its last cell to its
+// first, for rays against it, so that every ray goes up its list; four records
+// with an infinite node end each.
 struct alignas(32) RectCell {
   float x0, width, inv_width, ahead;
   int share;
 };
+constexpr int kRectEnd = 4;
+// records of one list, of an axis of `nodes` nodes
+__host__ __device__ constexpr int rect_list(int nodes) { return nodes - 1 + kRectEnd; }
 
 // Device view of one structured domain.
 struct DomainDev {
@@ -66,7 +71,7 @@ struct DomainDev {
   const float *bricks;    // vertex fields: bricked nodes
   const float *cells;     // element fields: linear cell values
   const RectCell *cell_rec;   // rectilinear: the axes' cells (see RectCell)
-  int rec_first[3];           // axis a's forward records, from cell_rec[rec_first[a]]
+  int rec_first[3];           // axis a's first list, from cell_rec[rec_first[a]]
   const float2 *brick_range;  // per-brick {min, max} of the field
   const uint8_t *brick_empty; // per-brick 1 = LUT alpha is 0 over its range
   const int *any_empty;       // 1 if any brick of this domain is empty
@@ -339,7 +344,7 @@ cudaError_t launch_march(const DomainDev *d_domains, const ViewDev &view,
                          const MarchParams &mp, const float4 *d_lut,
                          float4 *d_rgba, float *d_depth,
                          unsigned long long *d_samples, const Tuning &tuning,
-                         int mode, const int *d_order, cudaStream_t stream);
+                         int mode, bool long_steps, const int *d_order, cudaStream_t stream);
 // longest-first tile order for one view (gvr_march.cu): writes a permutation
 // of the view's kMarchTile tiles to d_order (one int per tile); d_keys holds
 // one word per tile of scratch and *d_top a word that is 0 between calls;

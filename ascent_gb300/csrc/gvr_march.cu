@@ -22,6 +22,9 @@ march_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
   __shared__ float s_state[kStateSlots * kThreads];
   float4 *lut = smem;
   DomainDev *doms = reinterpret_cast<DomainDev *>(smem + mp.lut_size);
+  // whether any domain has empty bricks under this transfer function; two loads,
+  // one after the other, on their way while the tables are copied
+  const bool mine = mp.skip_empty && threadIdx.x < mp.n_domains && *g_domains[threadIdx.x].any_empty;
   for (int i = threadIdx.x; i < mp.lut_size; i += kThreads) lut[i] = g_lut[i];
   {
     const int words = mp.n_domains * (int)(sizeof(DomainDev) / 4);
@@ -29,9 +32,7 @@ march_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
     uint32_t *dst = reinterpret_cast<uint32_t *>(doms);
     for (int i = threadIdx.x; i < words; i += kThreads) dst[i] = src[i];
   }
-  // whether any domain has empty bricks under this transfer function
-  const bool hidden = __syncthreads_or(mp.skip_empty && threadIdx.x < mp.n_domains &&
-                                       *g_domains[threadIdx.x].any_empty);
+  const bool hidden = __syncthreads_or(mine);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int px = tile_x * kTile + (warp % PX) * PW + (lane % PW);
@@ -67,7 +68,7 @@ constexpr int64_t kSmallFrame = 1536;   // tiles
 template <int PW, int UNROLL, int MINB>
 MarchFn pick() { return march_kernel<PW, UNROLL, MINB>; }
 
-MarchFn select(Tuning t, int mode, int64_t tiles)
+MarchFn select(Tuning t, int mode, int64_t tiles, bool long_steps)
 {
   t.packet_w = packet_width(t, mode, false);
   // Until a shape is set: small frames, whose few warps wait for their loads
@@ -86,12 +87,20 @@ MarchFn select(Tuning t, int mode, int64_t tiles)
     return m3 ? march_kernel<8, 1, 3, kMarchHex> : march_kernel<8, 1, 2, kMarchHex>;
   }
   // rectilinear domains keep three cells' records in registers besides the
-  // ray: 3 CTAs per SM whatever the tuning says (at 4 the loop spills and
-  // measured 3% slower); cell-centred ones take 4 (210 against 221 us on two
-  // domains of 160 x 144 x 121 cells at 1280 x 720)
-  if (mode == kMarchRect)
+  // ray, which 4 CTAs per SM spill: 502 against 464 us at 3 for the 242 x 200 x
+  // 174 nodes at 0.65 cells a step; with two cells a step and more the way from
+  // cell to cell waits for its loads, and 4 are faster (241^3 nodes at 1024^2:
+  // 618 and 622 us at one cell a step, 425 and 438 at two, 306 and 322 at four,
+  // 153 and 170 at 20). The tuning has no say.
+  if (mode == kMarchRect) {
+    if (long_steps)
+      return t.packet_w == 4 ? march_kernel<4, 2, 4, kMarchRect>
+                             : (t.packet_w == 16 ? march_kernel<16, 2, 4, kMarchRect> : march_kernel<8, 2, 4, kMarchRect>);
     return t.packet_w == 4 ? march_kernel<4, 2, 3, kMarchRect>
                            : (t.packet_w == 16 ? march_kernel<16, 2, 3, kMarchRect> : march_kernel<8, 2, 3, kMarchRect>);
+  }
+  // cell-centred ones take 4 (210 against 221 us on two domains of 160 x 144 x
+  // 121 cells at 1280 x 720)
   if (mode == kMarchCells)
     return t.packet_w == 4 ? march_kernel<4, 2, 4, kMarchCells>
                            : (t.packet_w == 16 ? march_kernel<16, 2, 4, kMarchCells> : march_kernel<8, 2, 4, kMarchCells>);
@@ -116,11 +125,11 @@ MarchFn select(Tuning t, int mode, int64_t tiles)
 cudaError_t launch_march(const DomainDev *d_domains, const ViewDev &view,
                          const MarchParams &mp, const float4 *d_lut, float4 *d_rgba,
                          float *d_depth, unsigned long long *d_samples, const Tuning &tuning,
-                         int mode, const int *d_order, cudaStream_t stream)
+                         int mode, bool long_steps, const int *d_order, cudaStream_t stream)
 {
   const size_t smem = sizeof(float4) * mp.lut_size + sizeof(DomainDev) * mp.n_domains;
   const int64_t tiles = (int64_t)((mp.width + kTile - 1) / kTile) * ((mp.height + kTile - 1) / kTile);
-  MarchFn fn = select(tuning, mode, tiles);
+  MarchFn fn = select(tuning, mode, tiles, long_steps);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(sizeof(float4) * kMaxLut + sizeof(DomainDev) * kMaxDomains));
   if (e != cudaSuccess) return e;

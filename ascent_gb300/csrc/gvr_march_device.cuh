@@ -115,19 +115,54 @@ __device__ __forceinline__ float div_by(float a, float b, float y)
   return fmaf(fmaf(-q, b, a), y, q);
 }
 
+// Steps of so many cells and more pass over no bricks: each holds four samples
+// at most (a frame of the 513^3 field at 100 samples, 5 cells a step, with its
+// publish: 534 us with, 475 us without; at a half cell a step the two are
+// within 2%).
+constexpr float kSkipCells = 2.f;
+
 // Along one axis of a rectilinear domain: where p lies past the node ahead,
-// step to the next cell (record c += step) and load its record, without a
-// branch.
-__device__ __forceinline__ void next_cell(RectCell &q, int &c, float p, int step, const RectCell *recs)
+// step to the ray's next cell and load its record, without a branch.
+__device__ __forceinline__ void next_cell(RectCell &q, int &c, float p, const RectCell *recs)
 {
   asm("{\n\t.reg .pred n;\n\t.reg .u64 at;\n\t"
       "setp.gt.f32 n, %6, %3;\n\t"
-      "@n add.s32 %5, %5, %7;\n\t"
-      "mad.wide.s32 at, %5, 32, %8;\n\t"
+      "@n add.s32 %5, %5, 1;\n\t"
+      "mad.wide.s32 at, %5, 32, %7;\n\t"
       "@n ld.global.nc.v4.f32 {%0, %1, %2, %3}, [at];\n\t"
       "@n ld.global.nc.s32 %4, [at + 16];\n\t}"
       : "+f"(q.x0), "+f"(q.width), "+f"(q.inv_width), "+f"(q.ahead), "+r"(q.share), "+r"(c)
-      : "f"(p), "r"(step), "l"(recs));
+      : "f"(p), "l"(recs));
+}
+
+// Along one axis: from a cell whose node ahead p may lie past, to the first
+// whose does not. Four nodes are compared at a time, since their loads need
+// nothing of each other, and the record is loaded for the cell found alone; the
+// lists end in four records that nothing lies past.
+__device__ __forceinline__ void far_cell(RectCell &q, int &c, float p, const RectCell *__restrict__ recs, unsigned warp)
+{
+  bool more = p > q.ahead;
+  if (!__any_sync(warp, more)) return;
+  const bool moves = more;
+  do {
+    if (more) {
+      const RectCell *at = recs + c;
+      const bool a = p > __ldg(&at[1].ahead), b = p > __ldg(&at[2].ahead);
+      const bool e = p > __ldg(&at[3].ahead), f = p > __ldg(&at[4].ahead);
+      // nodes ascend: as many are passed as there are comparisons that hold
+      c += min(1 + a + b + e + f, 4);
+      more = f;
+    }
+  } while (__any_sync(warp, more));
+  if (moves) {
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(recs + c));
+    q.x0 = v.x;
+    q.width = v.y;
+    q.inv_width = v.z;
+    q.ahead = v.w;
+    q.share = __ldg(&recs[c].share);
+  }
+  __syncwarp(warp);
 }
 
 // March one rectilinear domain (ELEM: a cell-centred field; SH: the brick
@@ -161,12 +196,11 @@ __device__ __noinline__ Partial march_rect(const DomainDev &dm, const Ray r, flo
   const bool skip = !ELEM && mp.skip_empty && *dm.any_empty;
   const RectCell *__restrict__ recs = dm.cell_rec;
   float sg[3], o[3], d[3];   // direction sign; origin and direction times it
-  int c[3], step[3];         // the cell's record in the ray's direction
+  int c[3];                  // the cell's record in the ray's direction
   RectCell q[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    step[a] = r.d[a] < 0.f ? -1 : 1;
-    sg[a] = (float)step[a];
+    sg[a] = r.d[a] < 0.f ? -1.f : 1.f;
     o[a] = sg[a] * r.o[a];
     d[a] = sg[a] * r.d[a];
     const RectCell *first = recs + dm.rec_first[a];
@@ -176,7 +210,7 @@ __device__ __noinline__ Partial march_rect(const DomainDev &dm, const Ray r, flo
       const int mid = (lo + hi) >> 1;
       if (__ldg(&first[mid].x0) <= p) lo = mid; else hi = mid;
     }
-    c[a] = dm.rec_first[a] + lo + (step[a] > 0 ? 0 : dm.dims[a] - 1);
+    c[a] = dm.rec_first[a] + (sg[a] > 0.f ? lo : rect_list(dm.dims[a]) + dm.dims[a] - 2 - lo);
     const float4 v = __ldg(reinterpret_cast<const float4 *>(recs + c[a]));
     q[a].x0 = v.x;
     q[a].width = v.y;
@@ -190,6 +224,16 @@ __device__ __noinline__ Partial march_rect(const DomainDev &dm, const Ray r, flo
   float4 col = make_float4(0.f, 0.f, 0.f, 0.f);   // ELEM: the cell's colour
   float lc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   int brick = -1;
+  bool hidden = false;   // the brick is empty
+  bool jumps = skip;
+  if (!ELEM && skip) {
+    // a brick of many cells to a step holds too few samples to jump over
+    float cells = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      cells = fmaxf(cells, fabsf(r.d[a]) * (float)(dm.dims[a] - 1) / (dm.hi[a] - dm.lo[a]));
+    jumps = cells * dt < kSkipCells;
+  }
   using At = typename std::conditional<ELEM, int64_t, int>::type;   // a bricked field holds < 2^31 floats
   At last = -1;
   const unsigned warp = __activemask();
@@ -200,13 +244,19 @@ __device__ __noinline__ Partial march_rect(const DomainDev &dm, const Ray r, flo
     if (!__any_sync(warp, !done)) return Partial{acc, k};
     t = done ? t0 : t;   // a lane that is done stays in its cells
     float p[3];
-    do {   // once, unless a step is longer than a cell
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        p[a] = fmaf(t, d[a], o[a]);
-        next_cell(q[a], c[a], p[a], step[a], recs);
+    for (int a = 0; a < 3; ++a) p[a] = fmaf(t, d[a], o[a]);
+    // steps of up to three cells one by one, longer ones four at a time
+    for (int hops = 0;; ++hops) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) next_cell(q[a], c[a], p[a], recs);
+      if (!__any_sync(warp, p[0] > q[0].ahead || p[1] > q[1].ahead || p[2] > q[2].ahead)) break;
+      if (hops == 2) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) far_cell(q[a], c[a], p[a], recs, warp);
+        break;
       }
-    } while (__any_sync(warp, p[0] > q[0].ahead || p[1] > q[1].ahead || p[2] > q[2].ahead));
+    }
     At at;
     if (ELEM) at = ((At)q[2].share * (dm.dims[1] - 1) + q[1].share) * (dm.dims[0] - 1) + q[0].share;
     else at = q[0].share + q[1].share + q[2].share;
@@ -219,38 +269,44 @@ __device__ __noinline__ Partial march_rect(const DomainDev &dm, const Ray r, flo
       } else {
         if (skip) {
           const int b = at / brick_floats(SH ? SH : bsh);
-          if (b != brick && dm.brick_empty[b]) {
-            // zero opacity over the whole brick: the samples up to one step
-            // before the ray leaves it are counted and jumped over, and the
-            // brick is looked up again at the next one
-            float texit = t1;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-              if (r.d[a] != 0.f) {
-                const int ba = (c[a] - dm.rec_first[a] - (step[a] > 0 ? 0 : dm.dims[a] - 1)) >> bsh;
-                const int e = step[a] > 0 ? min(((ba + 1) << bsh) - 1, dm.dims[a] - 2) : ba << bsh;
-                const RectCell *x = recs + dm.rec_first[a] + e;
-                texit = fminf(texit, ((step[a] > 0 ? __ldg(&x->ahead) : __ldg(&x->x0)) - r.o[a]) / r.d[a]);
-              }
-            }
-            taken = -max((int)floorf((texit - t0) / dt) - k, 1);   // negative: none of them is blended
-            last = -1;
-          } else {
+          if (b != brick) {
             brick = b;
+            hidden = dm.brick_empty[b];
           }
         }
-        const float *f = field + at;
-        lc[0] = __ldg(f);
-        lc[1] = __ldg(f + 1);
-        lc[2] = __ldg(f + bn);
-        lc[3] = __ldg(f + bn + 1);
-        lc[4] = __ldg(f + bn2);
-        lc[5] = __ldg(f + bn2 + 1);
-        lc[6] = __ldg(f + bn2 + bn);
-        lc[7] = __ldg(f + bn2 + bn + 1);
+        if (!hidden) {
+          const float *f = field + at;
+          lc[0] = __ldg(f);
+          lc[1] = __ldg(f + 1);
+          lc[2] = __ldg(f + bn);
+          lc[3] = __ldg(f + bn + 1);
+          lc[4] = __ldg(f + bn2);
+          lc[5] = __ldg(f + bn2 + 1);
+          lc[6] = __ldg(f + bn2 + bn);
+          lc[7] = __ldg(f + bn2 + bn + 1);
+        }
       }
     }
-    if (!ELEM) {
+    if (!ELEM && hidden) {
+      // zero opacity over the whole brick: the sample is counted alone, or with
+      // fine steps all samples up to one step before the ray leaves the brick
+      taken = -1;
+      if (jumps) {
+        float texit = t1;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          if (r.d[a] != 0.f) {
+            const int n = dm.dims[a] - 1, at0 = c[a] - dm.rec_first[a];
+            const bool up = sg[a] > 0.f;
+            const int ba = (up ? at0 : rect_list(n + 1) + n - 1 - at0) >> bsh;
+            const RectCell *x = recs + dm.rec_first[a] + (up ? min(((ba + 1) << bsh) - 1, n - 1) : ba << bsh);
+            texit = fminf(texit, __fdividef((up ? __ldg(&x->ahead) : __ldg(&x->x0)) - r.o[a], r.d[a]));
+          }
+        }
+        taken = -max((int)floorf(__fdividef(texit - t0, dt)) - k, 1);   // negative: none of them is blended
+      }
+    }
+    if (!ELEM && __any_sync(warp, !done && !hidden)) {
       float w[3];
 #pragma unroll
       for (int a = 0; a < 3; ++a)
@@ -808,11 +864,6 @@ __device__ __forceinline__ void finish_pixel(const ViewDev &view, const MarchPar
 // brick kept 18.4 of 32 lanes active and took 36.6 ms; this one keeps 26.3 and
 // takes 24.1. The 513^3 field in 8 domains at 1024^2: 1468 us with branches
 // out of the group's samples, 1433 us so.
-// Steps of so many cells and more pass over no bricks: each holds four samples
-// at most (a frame of the 513^3 field at 100 samples, 5 cells a step, with its
-// publish: 534 us with, 475 us without; at a half cell a step the two are
-// within 2%).
-constexpr float kSkipCells = 2.f;
 constexpr int kWalkDomains = 10;   // domains of a ray ordered at a time, 6 bits each in two words
 
 template <int UNROLL, int MODE, bool LIN>
