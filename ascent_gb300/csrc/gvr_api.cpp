@@ -1220,6 +1220,14 @@ static int render_one(gvr_scene *s, const gvr_camera *camera, const gvr_render_p
     }
     mp.canvas_rgba = d_rgba;
     mp.canvas_depth = d_depth;
+    for (int a = 0; a < 3; ++a) {
+      mp.box_lo[a] = INFINITY;
+      mp.box_hi[a] = -INFINITY;
+      for (const Domain &d : s->domains) {
+        mp.box_lo[a] = std::min(mp.box_lo[a], d.dev.lo[a]);
+        mp.box_hi[a] = std::max(mp.box_hi[a], d.dev.hi[a]);
+      }
+    }
   }
   const int *d_order = nullptr;
   const int64_t n_tiles = (int64_t)((p->width + kMarchTile - 1) / kMarchTile) *

@@ -154,6 +154,7 @@ struct MarchParams {
   // rays stop at its depth and partials blend over its colour
   const float4 *canvas_rgba = nullptr;
   const float *canvas_depth = nullptr;
+  float box_lo[3], box_hi[3];   // with a canvas: the box around all domains
 };
 
 // Reusable device buffers of one domain's field uploads: the staging copy

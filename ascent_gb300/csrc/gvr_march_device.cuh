@@ -43,7 +43,7 @@ struct Ray {
   float d[3];
 };
 
-__device__ __forceinline__ bool slab(const DomainDev &dm, const Ray &r, float &t0,
+__device__ __forceinline__ bool slab(const float *lo, const float *hi, const Ray &r, float &t0,
                                      float &t1)
 {
   float tmin = 0.f, tmax = FLT_MAX;
@@ -51,18 +51,23 @@ __device__ __forceinline__ bool slab(const DomainDev &dm, const Ray &r, float &t
   for (int a = 0; a < 3; ++a) {
     if (r.d[a] != 0.f) {
       const float inv = 1.f / r.d[a];
-      float ta = (dm.lo[a] - r.o[a]) * inv;
-      float tb = (dm.hi[a] - r.o[a]) * inv;
+      float ta = (lo[a] - r.o[a]) * inv;
+      float tb = (hi[a] - r.o[a]) * inv;
       if (ta > tb) { const float t = ta; ta = tb; tb = t; }
       tmin = fmaxf(tmin, ta);
       tmax = fminf(tmax, tb);
-    } else if (r.o[a] < dm.lo[a] || r.o[a] > dm.hi[a]) {
+    } else if (r.o[a] < lo[a] || r.o[a] > hi[a]) {
       return false;
     }
   }
   t0 = tmin;
   t1 = tmax;
   return tmax > tmin;
+}
+
+__device__ __forceinline__ bool slab(const DomainDev &dm, const Ray &r, float &t0, float &t1)
+{
+  return slab(dm.lo, dm.hi, r, t0, t1);
 }
 
 __device__ __forceinline__ float lerpf(float a, float b, float w)
@@ -729,7 +734,7 @@ __device__ __forceinline__ Ray pixel_ray(const ViewDev &view, const MarchParams 
 // Opaque canvas: the ray ends at the world point of the canvas depth
 // (MapCanvasToRays: pixel (i, j) at depth d unprojected from NDC
 // (2i/W - 1, 2j/H - 1, 2d - 1); FP64, as in the oracle). FLT_MAX where the
-// pixel's end lies past `far`, the ray's furthest exit from a domain, so that
+// pixel's end lies past `far`, at or past the ray's furthest exit from a domain, so that
 // it cuts nothing off: an FP32 estimate less its own error bound (each term of
 // a row within 16 units in the last place of the sum of the row's magnitudes)
 // shows that for the background and for surfaces behind the volume. The FP64
@@ -774,18 +779,15 @@ __device__ __noinline__ float canvas_ray_end(const ViewDev &view, const MarchPar
   return (float)sqrt(ex * ex + ey * ey + ez * ez);
 }
 
-// Where the canvas ends a ray, for the domains of `mask`; FLT_MAX without a
-// canvas and where no domain is hit.
-__device__ __forceinline__ float ray_end(const DomainDev *doms, uint64_t mask, const Ray &r, const ViewDev &view,
-                                         const MarchParams &mp, int px, int py)
+// Where the canvas ends a ray; FLT_MAX without a canvas, where the ray misses
+// the box around all domains, and where the canvas lies past that box. (The
+// furthest exit of the domains themselves costs a slab test each: 401 -> 484 us
+// for 48 small domains at 1280 x 769, before any sample.)
+__device__ __forceinline__ float ray_end(const Ray &r, const ViewDev &view, const MarchParams &mp, int px, int py)
 {
-  if (!mp.canvas_depth) return FLT_MAX;
-  float far = -1.f;
-  for (uint64_t m = mask; m; m &= m - 1) {
-    float t0, t1;
-    if (slab(doms[__ffsll((long long)m) - 1], r, t0, t1)) far = fmaxf(far, t1);
-  }
-  return far < 0.f ? FLT_MAX : canvas_ray_end(view, mp, px, py, far);
+  float t0, far;
+  if (!mp.canvas_depth || !slab(mp.box_lo, mp.box_hi, r, t0, far)) return FLT_MAX;
+  return canvas_ray_end(view, mp, px, py, far);
 }
 
 // The pixel's final value from its composited partial (have = whether any
@@ -875,7 +877,7 @@ __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_
   constexpr int BF = brick_floats(3);
   const Ray r = pixel_ray(view, mp, px, py);
   float *st = g_state + threadIdx.x;
-  st[7 * kThreads] = MODE == kMarchUniform ? FLT_MAX : ray_end(doms, mask, r, view, mp, px, py);
+  st[7 * kThreads] = MODE == kMarchUniform ? FLT_MAX : ray_end(r, view, mp, px, py);
   st[8 * kThreads] = __int_as_float(px);
   st[9 * kThreads] = __int_as_float(py);
   st[0 * kThreads] = 0.f;          // composited rgb
@@ -1113,7 +1115,7 @@ __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, 
   }
   int count = 0;
   const Ray r = pixel_ray(view, mp, px, py);
-  const float t_max = MODE == kMarchUniform ? FLT_MAX : ray_end(doms, mask, r, view, mp, px, py);
+  const float t_max = MODE == kMarchUniform ? FLT_MAX : ray_end(r, view, mp, px, py);
 
   // Compositing state that lives across the march of a domain is parked in
   // shared memory (one word per thread per slot, st[k * kThreads]), so the

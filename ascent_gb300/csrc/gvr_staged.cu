@@ -166,8 +166,7 @@ staged_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ V
   const int py = tile_y * kTile + (warp / PX) * PH + (lane / PW);
   const bool valid = px < mp.width && py < mp.height;
   const Ray r = pixel_ray(view, mp, valid ? px : 0, valid ? py : 0);
-  const float t_max =
-      valid ? ray_end(doms, mp.n_domains >= 64 ? ~0ull : (1ull << mp.n_domains) - 1ull, r, view, mp, px, py) : FLT_MAX;
+  const float t_max = valid ? ray_end(r, view, mp, px, py) : FLT_MAX;
   const float dt = mp.sample_dist;
   const float nm1 = (float)(mp.lut_size - 1);
 
@@ -578,8 +577,7 @@ layer_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
   }
 
   const Ray r = pixel_ray(view, mp, valid ? px : 0, valid ? py : 0);
-  const float t_max =
-      valid ? ray_end(doms, mp.n_domains >= 64 ? ~0ull : (1ull << mp.n_domains) - 1ull, r, view, mp, px, py) : FLT_MAX;
+  const float t_max = valid ? ray_end(r, view, mp, px, py) : FLT_MAX;
   const float dt = mp.sample_dist;
   const float nm1 = (float)(mp.lut_size - 1);
   float crgb[3] = {0.f, 0.f, 0.f}, ca = 0.f, cdepth = 0.f, covered = -FLT_MAX;
