@@ -62,6 +62,7 @@ struct DiffParams {
   int n_views;
   int lut_size;
   int n_seg;       // checkpoint segments per ray
+  double max_samples;  // of a ray, along the grid's diagonal
   int lut_copies;  // backward: LUT-gradient copies in global memory (CTA c uses c % copies)
   int64_t n_rays;  // views x height x width
   int packets;     // rays numbered by 8 x 4-pixel packets (see ray_number)
@@ -635,6 +636,7 @@ int diff_setup(const float *field, const int dims[3], const double origin[3],
                     ? 1.f / (params->scalar_max - params->scalar_min) : 0.f;
   const double max_samples = std::sqrt(diag) / params->sample_dist + 2.0;
   p.n_seg = (int)((max_samples + kDiffK - 1) / kDiffK);
+  p.max_samples = max_samples;
   p.lut_copies = 1;
   p.n_rays = (int64_t)n_views * params->width * params->height;
   p.packets = params->width % 8 == 0 && params->height % 4 == 0;
@@ -653,19 +655,25 @@ int packet_axis(const ViewDev &view, const DiffGrid &g)
 }
 
 // Copies the field's corner quads into scratch for the forward's views; false
-// where the field is read as it is. A copy costs 4.3 us per million nodes and
-// gains 0.7 to 1.05 us per million samples (counted at the diagonal's for every
-// ray), so each copy wants 8 samples a node: with 14, one view of a 128^3 field
-// at 256^2, the forward went from 102 to 72 us, with 8, one of 32^3 at 48^2,
-// from 18.1 to 15.6. Where there are not enough for a copy per axis all views
-// read the one along x. Not under capture, where the scratch would become part
-// of the graph, not beyond 1 GiB, and not where that is not to be had.
+// where the field is read as it is. In microseconds, a call with copies spends 14
+// more on the host (scratch and its end) and 5 a copy, and a copy 4.3 per
+// million nodes; the quads give back 0.55 per million samples (counted at the
+// diagonal's for every ray) where the samples' throughput bounds the frame and
+// 0.08 per sample of a ray where the longest ray does. Over 160 calls of 1 to
+// 16 views, 4 to 600 samples, 10^3 to 10^6 nodes, this takes the faster side or
+// one within some 10% of it; at 8 samples a node alone the copies cost calls with
+// short rays 15 to 25 of 80 us. With 14 samples a node, one view of a 128^3
+// field at 256^2, the forward went from 102 to 72 us. Where there are not enough
+// samples for a copy per axis all views read the one along x. Not under capture,
+// where the scratch would become part of the graph, not beyond 1 GiB, and not
+// where that is not to be had.
 bool make_quads(const float *field, const DiffGrid &g, const DiffViews &views, const DiffParams &p,
                 cudaStream_t st, DiffQuads &quads, float4 **scratch)
 {
   const int64_t nodes = (int64_t)g.dims[0] * g.dims[1] * g.dims[2];
-  const int64_t per_copy = p.n_rays * p.n_seg * kDiffK / (8 * nodes);   // copies that pay
-  if (per_copy < 1 || nodes > ((int64_t)1 << 26)) return false;
+  const double gain = std::max(0.55e-6 * (double)p.n_rays * p.max_samples, 0.08 * p.max_samples);
+  const auto pays = [&](int copies) { return gain > 14.0 + copies * (5.0 + 4.3e-6 * (double)nodes); };
+  if (!pays(1) || nodes > ((int64_t)1 << 26)) return false;
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
   if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
   bool wanted[3] = {};
@@ -675,7 +683,7 @@ bool make_quads(const float *field, const DiffGrid &g, const DiffViews &views, c
     copies += !wanted[quads.axis[v]];
     wanted[quads.axis[v]] = true;
   }
-  if (copies > per_copy || copies * nodes > ((int64_t)1 << 26)) {
+  if (!pays(copies) || copies * nodes > ((int64_t)1 << 26)) {
     std::fill(quads.axis, quads.axis + p.n_views, 0);
     wanted[0] = true;
     wanted[1] = wanted[2] = false;
