@@ -28,6 +28,7 @@ batch_kernel(const DomainDev *__restrict__ g_domains, const ViewDev *__restrict_
   __shared__ unsigned int s_item;
   __shared__ unsigned int s_mask[2];
   __shared__ float s_state[kStateSlots * kThreads];
+  const int empties = empties_of(mp);
   for (int i = threadIdx.x; i < mp.lut_size; i += kThreads) lut[i] = g_lut[i];
   {
     const int words = mp.n_domains * (int)(sizeof(DomainDev) / 4);
@@ -35,20 +36,7 @@ batch_kernel(const DomainDev *__restrict__ g_domains, const ViewDev *__restrict_
     uint32_t *dst = reinterpret_cast<uint32_t *>(doms);
     for (int i = threadIdx.x; i < words; i += kThreads) dst[i] = src[i];
   }
-  const bool hidden = __syncthreads_or(mp.skip_empty && threadIdx.x < mp.n_domains &&
-                                       *g_domains[threadIdx.x].any_empty);
-  // Of mostly empty scenes (half of 256 bricks looked at) the rays take their
-  // domains one by one: a ray's way through a domain is then mostly passing
-  // over bricks, which the lanes of a warp do together if they enter the domain
-  // together, and a tile's few domains are quickly searched for the next one.
-  // 64 views of 37 domains, 8-bit opacities: 12.9 ms in the one-loop walk, 9.4 so;
-  // opacities in floats, fewer empty bricks: 23.7 ms and 34.9.
-  bool by_domain = false;
-  if (MODE == kMarchUniform && hidden) {
-    const DomainDev &dm = doms[threadIdx.x % mp.n_domains];
-    const unsigned n = (unsigned)(dm.nbrick[0] * dm.nbrick[1] * dm.nbrick[2]);
-    by_domain = __syncthreads_count(dm.brick_empty[__umulhi(threadIdx.x * 2654435761u, n)]) >= kThreads / 2;
-  }
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_per_view = tiles_x * tiles_y;
   const long long total_tiles = (long long)tiles_per_view * n_views;
@@ -85,8 +73,8 @@ batch_kernel(const DomainDev *__restrict__ g_domains, const ViewDev *__restrict_
       if (px < mp.width && py < mp.height) {
         float4 out;
         float dep;
-        count += render_ray<UNROLL, MODE>(doms, mask, views[v], mp, lut, px, py, out, dep, s_state, hidden,
-                                          by_domain);
+        count += render_ray<UNROLL, MODE>(doms, mask, views[v], mp, lut, px, py, out, dep, s_state,
+                                          empties);
         const int64_t pix = (int64_t)v * pixels + (int64_t)py * mp.width + px;
         rgba[pix] = out;
         depth[pix] = dep;

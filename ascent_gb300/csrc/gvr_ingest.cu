@@ -388,6 +388,7 @@ struct EmptyJobs {
   uint8_t *empty[kMaxDomains];
   int *any_empty[kMaxDomains];
   int64_t first[kMaxDomains + 1];
+  int *n_empty;
   int n;
 };
 
@@ -425,7 +426,7 @@ empty_kernel(const __grid_constant__ EmptyJobs jobs, const float4 *__restrict__ 
   if (i1t == lut_size) before[lut_size] = (unsigned short)sum;   // the last threads all hold the total
   __syncthreads();
   const int64_t total = jobs.first[jobs.n];
-  int j = 0;
+  int j = 0, count = 0;
   for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < total;
        b += (int64_t)gridDim.x * blockDim.x) {
     while (b >= jobs.first[j + 1]) ++j;
@@ -442,6 +443,15 @@ empty_kernel(const __grid_constant__ EmptyJobs jobs, const float4 *__restrict__ 
     const bool e = before[i1 + 1] <= before[i0];   // also where the range is reversed (never)
     jobs.empty[j][l] = e;
     if (e) *jobs.any_empty[j] = 1;
+    count += e;
+  }
+  count = __reduce_add_sync(0xffffffffu, count);
+  __syncthreads();
+  if (lane == 0) warp_tot[warp] = count;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) count += warp_tot[w];
+    if (count) atomicAdd(jobs.n_empty, count);
   }
 }
 
@@ -645,12 +655,13 @@ cudaError_t launch_cells_field(const void *src, int dtype, int64_t stride,
 }
 
 cudaError_t launch_empty_bricks(int n, const float2 *const *brick_range, const int64_t *n_bricks,
-                                uint8_t *const *brick_empty, int *const *any_empty,
+                                uint8_t *const *brick_empty, int *const *any_empty, int *n_empty,
                                 const float4 *d_lut, int lut_size, int lut_filter,
                                 float scalar_min, float inv_range, cudaStream_t stream)
 {
   if (n > kMaxDomains || lut_size > kMaxLut) return cudaErrorInvalidValue;
   EmptyJobs jobs{};
+  jobs.n_empty = n_empty;
   for (int j = 0; j < n; ++j) {
     if (n_bricks[j] == 0) continue;
     jobs.range[jobs.n] = brick_range[j];

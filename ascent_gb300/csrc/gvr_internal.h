@@ -155,6 +155,10 @@ struct MarchParams {
   const float4 *canvas_rgba = nullptr;
   const float *canvas_depth = nullptr;
   float box_lo[3], box_hi[3];   // with a canvas: the box around all domains
+  // the scene's empty bricks, and from how many of them a frame passes over them
+  // and takes its domains one by one (see empties_of)
+  const int *n_empty;
+  int pass_from, by_domain_from;
 };
 
 // Reusable device buffers of one domain's field uploads: the staging copy
@@ -205,7 +209,7 @@ struct gvr_scene {
   gvr::DomainDev *d_domains = nullptr;   // device copy of the domain table
   int d_domains_cap = 0;
   float4 *d_lut = nullptr;               // LUT of the last render
-  int *d_any_empty = nullptr;            // per-domain empty-brick flags
+  int *d_any_empty = nullptr;            // per-domain empty-brick flags, then the number of empty bricks
   bool has_hex = false;
   gvr::Tuning tuning;
   unsigned long long *d_counters = nullptr;  // [0] samples, [1] staged waits given up
@@ -321,9 +325,10 @@ cudaError_t launch_cells_field(const void *src, int dtype, int64_t stride,
                                double range_out[2], Staging &stg,
                                cudaStream_t stream);
 // Classify the bricks of n domains' vertex fields against a transfer function
-// in one launch; *any_empty[j] becomes 1 when domain j has an empty brick.
+// in one launch; *any_empty[j] becomes 1 when domain j has an empty brick,
+// *n_empty grows by the empty bricks of all.
 cudaError_t launch_empty_bricks(int n, const float2 *const *brick_range, const int64_t *n_bricks,
-                                uint8_t *const *brick_empty, int *const *any_empty,
+                                uint8_t *const *brick_empty, int *const *any_empty, int *n_empty,
                                 const float4 *d_lut, int lut_size, int lut_filter,
                                 float scalar_min, float inv_range, cudaStream_t stream);
 

@@ -22,9 +22,7 @@ march_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
   __shared__ float s_state[kStateSlots * kThreads];
   float4 *lut = smem;
   DomainDev *doms = reinterpret_cast<DomainDev *>(smem + mp.lut_size);
-  // whether any domain has empty bricks under this transfer function; two loads,
-  // one after the other, on their way while the tables are copied
-  const bool mine = mp.skip_empty && threadIdx.x < mp.n_domains && *g_domains[threadIdx.x].any_empty;
+  const int empties = empties_of(mp);
   for (int i = threadIdx.x; i < mp.lut_size; i += kThreads) lut[i] = g_lut[i];
   {
     const int words = mp.n_domains * (int)(sizeof(DomainDev) / 4);
@@ -32,7 +30,7 @@ march_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
     uint32_t *dst = reinterpret_cast<uint32_t *>(doms);
     for (int i = threadIdx.x; i < words; i += kThreads) dst[i] = src[i];
   }
-  const bool hidden = __syncthreads_or(mine);
+  __syncthreads();
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int px = tile_x * kTile + (warp % PX) * PW + (lane % PW);
@@ -43,7 +41,7 @@ march_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
     const uint64_t all = mp.n_domains >= 64 ? ~0ull : ((1ull << mp.n_domains) - 1ull);
     float4 out;
     float dep;
-    count = render_ray<UNROLL, MODE>(doms, all, view, mp, lut, px, py, out, dep, s_state, hidden);
+    count = render_ray<UNROLL, MODE>(doms, all, view, mp, lut, px, py, out, dep, s_state, empties);
     const int64_t pix = (int64_t)py * mp.width + px;
     rgba[pix] = out;
     depth[pix] = dep;

@@ -120,10 +120,8 @@ __device__ __forceinline__ float div_by(float a, float b, float y)
   return fmaf(fmaf(-q, b, a), y, q);
 }
 
-// Steps of so many cells and more pass over no bricks: each holds four samples
-// at most (a frame of the 513^3 field at 100 samples, 5 cells a step, with its
-// publish: 534 us with, 475 us without; at a half cell a step the two are
-// within 2%).
+// Rectilinear domains: steps of so many cells and more do not jump to the end of
+// an empty brick, whose few samples are counted one by one.
 constexpr float kSkipCells = 2.f;
 
 // Along one axis of a rectilinear domain: where p lies past the node ahead,
@@ -872,7 +870,7 @@ constexpr int kWalkDomains = 10;   // domains of a ray ordered at a time, 6 bits
 template <int UNROLL, int MODE, bool LIN>
 __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_t mask, const ViewDev &view,
                                                   const MarchParams &mp, const float4 *lut, int px, int py,
-                                                  float4 &out, float &dep, float *g_state, bool any_hidden)
+                                                  float4 &out, float &dep, float *g_state, bool pass_over)
 {
   constexpr int BF = brick_floats(3);
   const Ray r = pixel_ray(view, mp, px, py);
@@ -995,10 +993,7 @@ __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_
         sy = dm.nbrick[0] * BF;
         sz = dm.nbrick[1] * sy;
         bricks = dm.bricks;
-        // steps of two cells and more: a brick holds so few samples that
-        // taking them costs less than passing over them
-        const float cells = dt * fmaxf(fabsf(B[0]), fmaxf(fabsf(B[1]), fabsf(B[2])));
-        hidden = any_hidden && cells < kSkipCells && *dm.any_empty ? d : -1;
+        hidden = pass_over && *dm.any_empty ? d : -1;
         k = 0;
         last_off = -1;
         brick = -1;
@@ -1087,6 +1082,17 @@ __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_
   return count;
 }
 
+// What a frame does at the empty bricks of uniform vertex domains (in 8^3-cell
+// bricks): take their samples like any others', which blend as nothing; pass over
+// them in the one-loop walk; pass over them in a loop per domain and brick, the
+// domains one by one. empty_limits has the limits and the reasons.
+enum { kEmptyTake = 0, kEmptyPass = 1, kEmptyByDomain = 2 };
+__device__ __forceinline__ int empties_of(const MarchParams &mp)
+{
+  const int n = mp.skip_empty ? *mp.n_empty : 0;
+  return n >= mp.by_domain_from ? kEmptyByDomain : n >= mp.pass_from ? kEmptyPass : kEmptyTake;
+}
+
 // MODE: what the scene holds, and so which march code its kernel carries. The
 // calls of the rectilinear and cell-centred loops cost a 64-register kernel
 // some 90 bytes of spills, which one of uniform vertex fields does without;
@@ -1094,15 +1100,15 @@ __device__ __forceinline__ int render_ray_unified(const DomainDev *doms, uint64_
 template <int UNROLL, int MODE>
 __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, const ViewDev &view,
                                           const MarchParams &mp, const float4 *lut, int px, int py,
-                                          float4 &out, float &dep, float *g_state, bool any_hidden,
-                                          bool by_domain = false)
+                                          float4 &out, float &dep, float *g_state, int empties)
 {
   if (MODE != kMarchHex && mask) {
     // domains that are all uniform vertex fields in 8^3-cell bricks, two or
     // more of them or one with empty bricks to pass over: the one-loop walk (a
     // single domain without has no crossing to wait at, and its own loop keeps
     // fewer values live: 1.39 against 1.49 ms on the 513^3 field as one domain)
-    bool walk = !by_domain && doms[__ffsll((long long)mask) - 1].bshift == 3 && ((mask & (mask - 1)) != 0 || any_hidden);
+    bool walk = empties != kEmptyByDomain && doms[__ffsll((long long)mask) - 1].bshift == 3 &&
+                ((mask & (mask - 1)) != 0 || empties == kEmptyPass);
     if (MODE != kMarchUniform)
       for (uint64_t m = mask; m; m &= m - 1) {
         const DomainDev &dm = doms[__ffsll((long long)m) - 1];
@@ -1110,8 +1116,8 @@ __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, 
       }
     if (walk)
       return mp.lut_filter == GVR_LUT_LINEAR
-                 ? render_ray_unified<UNROLL, MODE, true>(doms, mask, view, mp, lut, px, py, out, dep, g_state, any_hidden)
-                 : render_ray_unified<UNROLL, MODE, false>(doms, mask, view, mp, lut, px, py, out, dep, g_state, any_hidden);
+                 ? render_ray_unified<UNROLL, MODE, true>(doms, mask, view, mp, lut, px, py, out, dep, g_state, empties == kEmptyPass)
+                 : render_ray_unified<UNROLL, MODE, false>(doms, mask, view, mp, lut, px, py, out, dep, g_state, empties == kEmptyPass);
   }
   int count = 0;
   const Ray r = pixel_ray(view, mp, px, py);
@@ -1171,7 +1177,7 @@ __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, 
         MODE == kMarchUniform || (dm.kind == GVR_DOMAIN_UNIFORM && dm.assoc == GVR_ASSOC_VERTEX);
     if (MODE == kMarchHex && dm.kind == GVR_DOMAIN_HEX)
       count += march_hex(dm, r, bt0, bt1, mp, lut, thr, acc);
-    else if (uniform_vertex && !(mp.skip_empty && *dm.any_empty)) {
+    else if (uniform_vertex && (!(mp.skip_empty && *dm.any_empty) || (empties == kEmptyTake && dm.bshift == 3))) {
       if (mp.lut_filter == GVR_LUT_LINEAR)
         count += dm.bshift == 3 ? march_uniform<UNROLL, 3, true>(dm, r, bt0, bt1, mp, lut, thr, acc)
                : dm.bshift == 2 ? march_uniform<UNROLL, 2, true>(dm, r, bt0, bt1, mp, lut, thr, acc)
@@ -1181,10 +1187,11 @@ __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, 
                : dm.bshift == 2 ? march_uniform<UNROLL, 2, false>(dm, r, bt0, bt1, mp, lut, thr, acc)
                                 : march_uniform<UNROLL, 4, false>(dm, r, bt0, bt1, mp, lut, thr, acc);
     } else if (uniform_vertex) {
-      // 8^3-cell bricks come here next to other kinds of domains and by_domain
-      count += (MODE != kMarchUniform || by_domain) && dm.bshift == 3 ? march_bricks<UNROLL, 3>(dm, r, bt0, bt1, mp, lut, thr, acc)
-             : dm.bshift == 2                          ? march_bricks<UNROLL, 2>(dm, r, bt0, bt1, mp, lut, thr, acc)
-                                                       : march_bricks<UNROLL, 4>(dm, r, bt0, bt1, mp, lut, thr, acc);
+      // 8^3-cell bricks come here next to other kinds of domains and domain by domain
+      count += (MODE != kMarchUniform || empties == kEmptyByDomain) && dm.bshift == 3
+                   ? march_bricks<UNROLL, 3>(dm, r, bt0, bt1, mp, lut, thr, acc)
+                   : dm.bshift == 2 ? march_bricks<UNROLL, 2>(dm, r, bt0, bt1, mp, lut, thr, acc)
+                                    : march_bricks<UNROLL, 4>(dm, r, bt0, bt1, mp, lut, thr, acc);
     }
     else {
       Partial part;

@@ -562,7 +562,7 @@ layer_kernel(const DomainDev *__restrict__ g_domains, const __grid_constant__ Vi
       const uint64_t all = mp.n_domains >= 64 ? ~0ull : ((1ull << mp.n_domains) - 1ull);
       float4 out;
       float dep;
-      count = render_ray<1, kMarchCells>(doms, all, view, mp, lut, px, py, out, dep, s_state, true);
+      count = render_ray<1, kMarchCells>(doms, all, view, mp, lut, px, py, out, dep, s_state, empties_of(mp));
       const int64_t pix = (int64_t)py * mp.width + px;
       rgba[pix] = out;
       depth[pix] = dep;
