@@ -748,7 +748,8 @@ size_t sorted_bytes(int64_t n)
 }
 
 // Whether the slots serve: their places are read for every pixel, and take 32
-// bytes of scratch each.
+// bytes of scratch each (40 a pixel and 12 a record in all, the histogram path
+// 16 and 12: where the larger amount is not to be had, that path is taken).
 bool use_slots(int64_t n, int64_t r) { return r <= 2 * n; }
 
 size_t slot_bytes(int64_t n, int64_t r)
@@ -913,9 +914,10 @@ extern "C" int gvr_composite_partials(const gvr_partial *partials, int64_t n, gv
     const int lo = (int)(hm[0] ^ 0x80000000u), hi = (int)(hm[1] ^ 0x80000000u);
     const int64_t r = (int64_t)hi - lo + 1;
     const bool dense = r <= 2 * n + 65536 && r < ((int64_t)1 << 31);
-    const bool slots = dense && use_slots(n, r);
-    const size_t bytes = slots ? slot_bytes(n, r) : dense ? dense_bytes(n, r) : sorted_bytes(n);
-    CP_TRY(scratch_alloc((void **)&arena.base, bytes, st), "allocate scratch");
+    bool slots = dense && use_slots(n, r);
+    CP_TRY(slots ? scratch_alloc((void **)&arena.base, slot_bytes(n, r), dense_bytes(n, r), &slots, st)
+                 : scratch_alloc((void **)&arena.base, dense ? dense_bytes(n, r) : sorted_bytes(n), st),
+           "allocate scratch");
     totals = arena.take<uint32_t>(2);
     // the range was measured, so no record is outside it: mm[0] serves as
     // the (unused) flag word
@@ -960,8 +962,9 @@ extern "C" int gvr_composite_partials_async(const gvr_partial *partials, int64_t
     return e == cudaSuccess ? GVR_OK : cuda_error(e, "composite");
   }
   Arena arena;
-  const bool slots = use_slots(n, r);
-  e = scratch_alloc((void **)&arena.base, slots ? slot_bytes(n, r) : dense_bytes(n, r), st);
+  bool slots = use_slots(n, r);
+  e = slots ? scratch_alloc((void **)&arena.base, slot_bytes(n, r), dense_bytes(n, r), &slots, st)
+            : scratch_alloc((void **)&arena.base, dense_bytes(n, r), st);
   if (e != cudaSuccess) return cuda_error(e, "allocate scratch");
   uint32_t *totals = arena.take<uint32_t>(2);
   if (slots) {

@@ -276,6 +276,8 @@ void make_view(const gvr_camera &cam, int width, int height, ViewDev *v);
 // device (kept between calls, unlike the default pool's); free it with
 // cudaFreeAsync
 cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
+// `bytes` where they are to be had (*all), else `least`
+cudaError_t scratch_alloc(void **ptr, size_t bytes, size_t least, bool *all, cudaStream_t stream);
 
 // Device memory of scenes and of their builds, from a second pool of this
 // library: usable at once on any stream. device_free waits for the device

@@ -177,6 +177,15 @@ cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream)
   return cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
 }
 
+cudaError_t scratch_alloc(void **ptr, size_t bytes, size_t least, bool *all, cudaStream_t stream)
+{
+  cudaError_t e = scratch_alloc(ptr, bytes, stream);
+  *all = e == cudaSuccess;
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  return scratch_alloc(ptr, least, stream);
+}
+
 }  // namespace gvr
 
 int gvr_scratch_trim(int device, uint64_t keep_bytes, uint64_t *reserved_out)

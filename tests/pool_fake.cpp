@@ -201,10 +201,27 @@ static void out_of_memory()
   CHECK(held == 0);
 }
 
+// The larger amount where it fits, the smaller where only that does.
+static void either_amount()
+{
+  void *a, *s;
+  bool all = false;
+  CHECK(scratch_alloc(&s, 600000, 100000, &all, nullptr) == cudaSuccess && all);
+  CHECK(cudaFreeAsync(s, nullptr) == cudaSuccess);
+  CHECK(device_alloc(&a, 700000) == cudaSuccess);
+  CHECK(scratch_alloc(&s, 600000, 100000, &all, nullptr) == cudaSuccess && !all && last == cudaSuccess);
+  CHECK(blocks[s].bytes == 100000);
+  void *t;
+  CHECK(scratch_alloc(&t, 600000, 500000, &all, nullptr) == cudaErrorMemoryAllocation && !all);
+  last = cudaSuccess;
+  CHECK(cudaFreeAsync(s, nullptr) == cudaSuccess && device_free(a) == cudaSuccess);
+}
+
 int main()
 {
   for (int then = 0; then < 3; ++then) refused_wait(then);
   refused_allocation();
   out_of_memory();
+  either_amount();
   return checks_failed != 0;
 }
