@@ -523,6 +523,7 @@ static int add_structured(gvr_scene *s, int kind, const int dims[3], const doubl
         f.x0 = x0;
         f.width = x1 - x0;
         f.inv_width = 1.0f / f.width;
+        if (!(f.width >= kByReciprocal[0] && f.width < kByReciprocal[1])) d.dev.divide = 1;
         f.ahead = i + 1 < n ? x1 : INFINITY;
         f.share = assoc == GVR_ASSOC_ELEMENT
                       ? i : (int)((i >> sh) * of_brick + (i & (brick_cells(sh) - 1)) * in_brick);

@@ -55,6 +55,8 @@ struct alignas(32) RectCell {
   int share;
 };
 constexpr int kRectEnd = 4;
+// Widths whose weights are taken by the reciprocal (see div_by).
+constexpr float kByReciprocal[2] = {0x1p-64f, 0x1p64f};
 // records of one list, of an axis of `nodes` nodes
 __host__ __device__ constexpr int rect_list(int nodes) { return nodes - 1 + kRectEnd; }
 
@@ -72,6 +74,7 @@ struct DomainDev {
   const float *cells;     // element fields: linear cell values
   const RectCell *cell_rec;   // rectilinear: the axes' cells (see RectCell)
   int rec_first[3];           // axis a's first list, from cell_rec[rec_first[a]]
+  int divide;                 // rectilinear: 1 if a cell's width is outside kByReciprocal
   const float2 *brick_range;  // per-brick {min, max} of the field
   const uint8_t *brick_empty; // per-brick 1 = LUT alpha is 0 over its range
   const int *any_empty;       // 1 if any brick of this domain is empty

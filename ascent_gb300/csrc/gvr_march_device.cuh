@@ -113,7 +113,10 @@ __device__ __forceinline__ float4 lut_color(const float4 *lut, const MarchParams
 // a / b from y = RN(1 / b): the product a y corrected by its residual
 // (Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000", 1990). Three operations against the eight or so and the
-// branch of a general division; b is a cell's width and y is kept with it.
+// branch of a general division; b is a cell's width and y is kept with it. The
+// quotient is the divide's where 1 / b is a normal number and the residual, down
+// to 2^-46 a, keeps its last bit: for b in kByReciprocal and a down to 2^-38 b.
+// Domains with other cells divide.
 __device__ __forceinline__ float div_by(float a, float b, float y)
 {
   const float q = a * y;
@@ -189,7 +192,7 @@ __device__ __forceinline__ void far_cell(RectCell &q, int &c, float p, const Rec
 // from three cells, 460 us. Not inlined, so that its registers do not weigh on
 // the kernels' uniform-grid loop; the ray comes by value and the result goes
 // back by value, so nothing is kept in local memory for the call.
-template <bool ELEM, int SH>
+template <bool ELEM, int SH, bool DIVIDE = false>
 __device__ __noinline__ Partial march_rect(const DomainDev &dm, const Ray r, float t0, float t1,
                                            const MarchParams &mp, const float4 *lut, float thr)
 {
@@ -234,7 +237,7 @@ __device__ __noinline__ Partial march_rect(const DomainDev &dm, const Ray r, flo
     float cells = 0.f;
 #pragma unroll
     for (int a = 0; a < 3; ++a)
-      cells = fmaxf(cells, fabsf(r.d[a]) * (float)(dm.dims[a] - 1) / (dm.hi[a] - dm.lo[a]));
+      cells = fmaxf(cells, __fdividef(fabsf(r.d[a]) * (float)(dm.dims[a] - 1), dm.hi[a] - dm.lo[a]));
     jumps = cells * dt < kSkipCells;
   }
   using At = typename std::conditional<ELEM, int64_t, int>::type;   // a bricked field holds < 2^31 floats
@@ -313,7 +316,8 @@ __device__ __noinline__ Partial march_rect(const DomainDev &dm, const Ray r, flo
       float w[3];
 #pragma unroll
       for (int a = 0; a < 3; ++a)
-        w[a] = __saturatef(div_by(fmaf(sg[a], p[a], -q[a].x0), q[a].width, q[a].inv_width));
+        w[a] = __saturatef(DIVIDE ? fmaf(sg[a], p[a], -q[a].x0) / q[a].width
+                                  : div_by(fmaf(sg[a], p[a], -q[a].x0), q[a].width, q[a].inv_width));
       const float c00 = lerpf(lc[0], lc[1], w[0]);
       const float c10 = lerpf(lc[2], lc[3], w[0]);
       const float c01 = lerpf(lc[4], lc[5], w[0]);
@@ -1197,6 +1201,7 @@ __device__ __forceinline__ int render_ray(const DomainDev *doms, uint64_t mask, 
       Partial part;
       if (MODE >= kMarchRect && dm.kind == GVR_DOMAIN_RECTILINEAR)
         part = dm.assoc == GVR_ASSOC_ELEMENT ? march_rect<true, 0>(dm, r, bt0, bt1, mp, lut, thr)
+               : dm.divide                  ? march_rect<false, 0, true>(dm, r, bt0, bt1, mp, lut, thr)
                : dm.bshift == 3             ? march_rect<false, 3>(dm, r, bt0, bt1, mp, lut, thr)
                                              : march_rect<false, 0>(dm, r, bt0, bt1, mp, lut, thr);
       else
