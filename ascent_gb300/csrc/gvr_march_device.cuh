@@ -189,7 +189,8 @@ __device__ __forceinline__ void far_cell(RectCell &q, int &c, float p, const Rec
 // return per lane, 15 to 18 of 32 lanes active, 710-983 us; without the
 // branches and with the votes 532 us; with a record per direction and a
 // brick's number taken from the offset (a division by a constant) instead of
-// from three cells, 460 us. Not inlined, so that its registers do not weigh on
+// from three cells, 498 us; with every ray going up a list of its own direction,
+// 486 us. Not inlined, so that its registers do not weigh on
 // the kernels' uniform-grid loop; the ray comes by value and the result goes
 // back by value, so nothing is kept in local memory for the call.
 template <bool ELEM, int SH, bool DIVIDE = false>
@@ -736,14 +737,16 @@ __device__ __forceinline__ Ray pixel_ray(const ViewDev &view, const MarchParams 
 // Opaque canvas: the ray ends at the world point of the canvas depth
 // (MapCanvasToRays: pixel (i, j) at depth d unprojected from NDC
 // (2i/W - 1, 2j/H - 1, 2d - 1); FP64, as in the oracle). FLT_MAX where the
-// pixel's end lies past `far`, at or past the ray's furthest exit from a domain, so that
-// it cuts nothing off: an FP32 estimate less its own error bound (each term of
+// pixel's end lies past `far`, at or past the ray's furthest exit from a domain,
+// so that it cuts nothing off: an FP32 estimate less its own error bound (each term of
 // a row within 16 units in the last place of the sum of the row's magnitudes)
 // shows that for the background and for surfaces behind the volume. The FP64
 // pipe issues a warp in some 16 cycles, and the hundred or so FP64 operations
-// of the plain form for every pixel were more than half of a 1280 x 720 frame
-// (208 us; 140 us with the bound, 12 multiply-adds on matrices that hold the
-// NDC map, and one division).
+// of the plain form for every pixel were more than half of a 1280 x 720 frame;
+// the bound takes 12 multiply-adds on matrices that hold the NDC map, and one
+// division. Four cell-centred domains of 160 x 144 x 121 cells in all, in front
+// of a canvas: 277 us with the plain form and a sample at a time, 163 us so and
+// with four in flight.
 __device__ __noinline__ float canvas_ray_end(const ViewDev &view, const MarchParams &mp, int px, int py,
                                              float far)
 {
@@ -866,8 +869,8 @@ __device__ __forceinline__ void finish_pixel(const ViewDev &view, const MarchPar
 // Bound by instructions and, at a sample per half cell and pixel, as much by
 // L1 wavefronts (75% of their peak, 33 a sample of a warp). 64 views at 512^2
 // of 37 domains, whose rays cross some six of them: a loop per domain and per
-// brick kept 18.4 of 32 lanes active and took 36.6 ms; this one keeps 26.3 and
-// takes 24.1. The 513^3 field in 8 domains at 1024^2: 1468 us with branches
+// brick kept 18.4 of 32 lanes active and took 36.6 ms; this one keeps 27.9 and
+// takes 23.7. The 513^3 field in 8 domains at 1024^2: 1468 us with branches
 // out of the group's samples, 1433 us so.
 constexpr int kWalkDomains = 10;   // domains of a ray ordered at a time, 6 bits each in two words
 
