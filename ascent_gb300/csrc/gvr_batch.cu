@@ -100,7 +100,7 @@ using BatchFn = void (*)(const DomainDev *, const ViewDev *, const int4 *, const
 
 BatchFn select_batch(Tuning t, int mode)
 {
-  t.packet_w = packet_width(t, mode, true);
+  t.packet_w = packet_width(t, mode, true, 0);
   if (mode == kMarchHex) return t.packet_w == 4 ? batch_kernel<4, 1, 2, kMarchHex> : batch_kernel<8, 1, 2, kMarchHex>;
   if (mode == kMarchRect)
     return t.packet_w == 4 ? batch_kernel<4, 2, 3, kMarchRect>

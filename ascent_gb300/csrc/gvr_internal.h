@@ -102,15 +102,21 @@ struct Tuning {
                             // 1 = longest-first by the view's estimated tile cost
 };
 
+constexpr int64_t kSmallFrame = 1536;   // tiles
+
 // The packet width of a scene that none was set for. 4-wide packets are 1 to
 // 8% faster than 8-wide ones over seven views of the 513^3 field at 1024^2
 // (1442 -> 1390 us at azimuth 30, elevation 20; equal seen along an axis) and
-// of 8M hexahedra (4999 -> 4729 us), and within 3% of them on smaller frames.
+// within 3% of them on smaller frames. Of hexahedra, 8M at 1024^2 take 4570 us 4
+// wide and 4651 8 wide; below kSmallFrame tiles, where a few warps of long rays
+// make the frame, 15 meshes and views take 4% less 8 wide on average (76 x 27 x
+// 150 cells at 491 x 304: 391 us for 496; at the other end 340 for 322).
 // Rectilinear frames are 1 to 7% faster 8 wide in four of the seven, and 64
 // batched views of 37 domains 3% (24.1 against 24.8 ms).
-inline int packet_width(const Tuning &t, int mode, bool batch)
+inline int packet_width(const Tuning &t, int mode, bool batch, int64_t tiles)
 {
-  return t.packet_w ? t.packet_w : (batch || mode == kMarchRect ? 8 : 4);
+  if (t.packet_w) return t.packet_w;
+  return batch || mode == kMarchRect || (mode == kMarchHex && tiles < kSmallFrame) ? 8 : 4;
 }
 
 // Front-to-back order of a scene's domains for one view (staged march).

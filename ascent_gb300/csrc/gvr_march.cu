@@ -61,14 +61,12 @@ namespace {
 using MarchFn = void (*)(const DomainDev *, const ViewDev, const MarchParams, const float4 *,
                          float4 *, float *, unsigned long long *, const int *);
 
-constexpr int64_t kSmallFrame = 1536;   // tiles
-
 template <int PW, int UNROLL, int MINB>
 MarchFn pick() { return march_kernel<PW, UNROLL, MINB>; }
 
 MarchFn select(Tuning t, int mode, int64_t tiles, bool long_steps)
 {
-  t.packet_w = packet_width(t, mode, false);
+  t.packet_w = packet_width(t, mode, false, tiles);
   // Until a shape is set: small frames, whose few warps wait for their loads
   // more than for each other, take four samples per iteration at 3 CTAs per SM
   // (10 to 14% faster at 80 to 1200 tiles, 46.3 -> 41.8 us for the 64^3 field at

@@ -276,7 +276,8 @@ GVR_API int gvr_scene_update_fields(gvr_scene *scene, int n, const int *domain_i
 GVR_API int gvr_scene_num_domains(const gvr_scene *scene, int *n);
 
 /* Launch shape of the scene's march kernel: pixel packet width per warp
- * (4, 8 or 16; the packet is 32 rays; by the scene until one is set), samples located
+ * (4, 8 or 16; the packet is 32 rays; by the scene and the frame's size until
+ * one is set), samples located
  * per loop iteration (1 to 4; 16-wide packets at most 3, and 3 only with
  * min_blocks 4; 3 and 4 run as 4 with min_blocks 3 and as 2 otherwise, on the
  * batch path as 2) and CTAs per SM targeted by the register budget (3 or 4).
